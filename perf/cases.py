@@ -55,15 +55,15 @@ def listed() -> list[dict]:
         # a solvent box of an everyday study, flexible water, SPME, odd size
         dict(name="water-9k-nvt", kind="water", n_mol=3001, steps=50, thermostat="nose-hoover",
              profile="phys", precision="mixed"),
-        # the headline workload
+        # the headline workload (64^3 mesh)
         dict(name="water-30k-nvt", kind="water", n_mol=10000, steps=50, thermostat="nose-hoover",
              profile="phys", precision="mixed"),
         # the same box on the all-FP64 path (a reference run to trust the mixed one by)
         dict(name="water-30k-fp64", kind="water", n_mol=10000, steps=20,
              thermostat="nose-hoover", profile="phys", precision="fp64"),
-        # the large box, constant pressure
+        # the large box, constant pressure (192^3 mesh)
         dict(name="water-750k-npt", kind="water", n_mol=250000, steps=30, thermostat="berendsen",
-             barostat="berendsen", profile="phys", precision="mixed"),
+             barostat="berendsen", spacing=0.1019, profile="phys", precision="mixed"),
         # a molecular melt without charges: bonds, angles, dihedrals, exclusions
         dict(name="decane-4k-nvt", kind="decane", n_chains=400, steps=100,
              thermostat="berendsen", profile="phys", precision="mixed"),
@@ -172,7 +172,7 @@ def _argon(cells, seed):
     return _base(p, cells * a, np.full(len(p), 39.948), 1.0, 0.002, 120.0, rng)
 
 
-def _water(n_mol, seed, rigid=False):
+def _water(n_mol, seed, rigid=False, spacing=0.1045):
     rng = np.random.default_rng(seed)
     box = (n_mol / 33.4) ** (1.0 / 3.0)
     o, a = _lattice(n_mol, box)
@@ -192,7 +192,7 @@ def _water(n_mol, seed, rigid=False):
     s = _base(pos, box, np.tile([15.9994, 1.008, 1.008], n_mol), 1.0, 0.002 if rigid else 0.0005, 300.0,
               rng, charge=np.tile([-0.8476, 0.4238, 0.4238], n_mol), types=np.tile(np.array([1, 0, 0], np.int32), n_mol),
               sig=np.array([[1.0, 1.0], [1.0, 0.3166]]), eps=np.array([[0.0, 0.0], [0.0, 0.650]]),
-              coulomb="pme", spacing=box / math.ceil(box / 0.1045 - 1e-9),
+              coulomb="pme", spacing=spacing,
               bonds=oh, bond_k=np.full(2 * n_mol, 345000.0), bond_r0=np.full(2 * n_mol, 0.1),
               angles=np.stack([m + 1, m, m + 2], 1), angle_k=np.full(n_mol, 383.0),
               angle_t0=np.full(n_mol, th), excl=hh)
@@ -245,7 +245,7 @@ def _system(case, seed):
     elif case["kind"] == "argon":
         s = _argon(case["cells"], seed)
     elif case["kind"] == "water":
-        s = _water(case["n_mol"], seed, bool(case.get("rigid")))
+        s = _water(case["n_mol"], seed, bool(case.get("rigid")), case.get("spacing", 0.1045))
     else:
         s = _decane(case["n_chains"], seed)
     s["thermostat"] = case.get("thermostat", "none")
@@ -380,9 +380,9 @@ def _step_work(s_or_n, rho=None, charged=False, rc=1.0, terms=0.0, mesh=0):
     return dict(bytes=144.0 * n + (16.0 * mesh ** 3 if mesh else 0) + 40 * terms, flops=flops)
 
 
-def _kind_work(kind, n, rho):
+def _kind_work(kind, n, rho, spacing=0.1045):
     if kind == "water":
-        mesh = math.ceil((n / 3 / 33.4) ** (1 / 3) / 0.1045 - 1e-9)
+        mesh = max(8, int((n / 3 / 33.4) ** (1 / 3) / spacing + 0.5))
         return _step_work(n, 100.2, True, 1.0, 2.0 * n, mesh)
     if kind == "decane":
         return _step_work(n, 27.0, False, 0.9875, 6.2 * n)
@@ -404,7 +404,7 @@ def work(case):
         return {k: case["n_jobs"] * steps * (0.7 * a[k] + 0.3 * w[k]) for k in a}
     n = {"lj": case.get("n"), "argon": 4 * case.get("cells", 0) ** 3, "water": 3 * case.get("n_mol", 0),
          "decane": 10 * case.get("n_chains", 0)}[kind]
-    w = _kind_work(kind, n, case.get("rho"))
+    w = _kind_work(kind, n, case.get("rho"), case.get("spacing", 0.1045))
     return {k: v * (1 if case.get("single") else case["steps"]) for k, v in w.items()}
 
 
