@@ -190,7 +190,11 @@ class Batch {
     bool any_pme_ = false, any_baro_ = false, any_narrow_ = false, any_ref_lj_ = false, any_andersen_ref_ = false,
          any_andersen_phys_ = false;
     std::map<int, std::pair<cufftHandle, cufftHandle>> plans_;
-    cudaGraphExec_t graph_ = nullptr;
+    cudaGraphExec_t graph_ = nullptr;       // one step
+    cudaGraphExec_t graph_many_ = nullptr;  // kManySteps steps (tables that keep running)
+    long long steps_run_ = 0;               // steps launched from graph_ or graph_many_
+    int capture_steps(int n, cudaGraphExec_t* out);
+    void drop_graphs();
     bool packed_ = false;
     // a list build timed out: its sort and list buffers are in an unknown
     // state, so no further device work is issued on this table
