@@ -1180,25 +1180,32 @@ int Batch::pack() {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         const TuneKey key = tune_key(device_, fp64_, any_pme_, dev_.n_atoms, opt_.nb_form, density_);
         auto it = g_tune.find(key);
-        if (it == g_tune.end()) {
-            // a table of a size not tuned yet takes the shape tuned for the
-            // nearest size of the same kind, so a serving loop whose table size
-            // changes with every admission tunes once, not at every rebuild
-            int best = 1 << 30;
-            for (auto jt = g_tune.begin(); jt != g_tune.end(); ++jt) {
-                const TuneKey& k = jt->first;
-                if (k.device != key.device || k.fp64 != key.fp64 || k.pme != key.pme || k.forced != key.forced)
-                    continue;
-                const int dist = 4 * std::abs(k.dens - key.dens) + std::abs(k.bucket - key.bucket);
-                if (dist < best) {
-                    best = dist;
-                    it = jt;
-                }
-            }
-        }
-        tuned_ = fp64_ || it != g_tune.end();
         nb_form_ = uses_clusters() ? NB_CLUSTER8 : NB_CHUNK32;
-        nb_blocks_per_sm_ = (it != g_tune.end()) ? it->second.bps : ((any_pme_ || nb_form_ == NB_CLUSTER8) ? 2 : 3);
+        // The pair kernel's shape follows from the list: one warp per chunk as
+        // far as its registers allow (4 blocks per SM for LJ only, 3 with
+        // real-space Coulomb), one block fewer where bonded terms or a PME chain
+        // run beside it in the room it leaves.  lj 20k (3,669 chunks) 14.2 ->
+        // 11.1 us, a 64-replica batch 276 -> 200 us per launch at 4 blocks
+        // against 2; decane 4k (1,161 chunks, bonded terms 10 us beside) a step
+        // of 33.0 us at 2 blocks, 37.7 at 4; water 30k 126 us at 2 against 142
+        // at 3.  Above 400,000 atoms every kernel fills the GPU by itself and
+        // the chain gains nothing from running beside (750k: 2.79 ms at 2
+        // blocks, 2.74 at 3).  A table with a PME chain measures the other
+        // shapes too (autotune).
+        rule_bps_ = !fp64_ && !any_pme_ && nb_form_ == NB_CHUNK32;
+        tuned_ = fp64_ || it != g_tune.end();
+        if (nb_form_ == NB_CLUSTER8) {
+            nb_blocks_per_sm_ = 2;
+        } else {
+            long long chunks = 0;
+            for (int k = 0; k < R; ++k) chunks += n_chunks_built_[k];
+            const long long per_block = 8LL * n_sm_;
+            const bool beside = dev_.n_bonds + dev_.n_excl > 0 || any_pme_;
+            const int most = (dev_.any_coul ? 3 : 4) - (beside && dev_.n_atoms < 400000 ? 1 : 0);
+            nb_blocks_per_sm_ =
+                static_cast<int>(std::min<long long>(most, std::max<long long>(1, (chunks + per_block - 1) / per_block)));
+        }
+        if (!rule_bps_ && it != g_tune.end()) nb_blocks_per_sm_ = it->second.bps;
     }
     packed_ = true;
     graph_dirty_ = true;
@@ -1370,11 +1377,12 @@ void Batch::drop_graphs() {
 // 94, water 30k 142 -> 125; eight and sixteen gained nothing more.  Above
 // kManyAtoms the gap does not count and the later steps' persistent pair
 // blocks got in the way of the mesh kernels (750k: 2.76 -> 2.80 ms).
-// Capturing and instantiating costs 0.3-0.5 ms, about what it saves in 64
-// steps, so it waits until a table has run that many: a served table that is
-// rebuilt every few calls keeps the one-step graph.
+// Capturing and instantiating costs 0.3-1 ms, what it saves in 60 to 300
+// steps, so it waits until a table has run 256: a served table that is rebuilt
+// every few calls keeps the one-step graph (at 64 a served wave of 8 jobs took
+// 120.5 ms against 116.0).
 constexpr int kManySteps = 4;
-constexpr int kManyAfter = 64;
+constexpr int kManyAfter = 256;
 constexpr int kManyAtoms = 400000;
 
 int Batch::run_steps(int n) {
@@ -1413,7 +1421,7 @@ int Batch::run_steps(int n) {
         CK(cudaGetLastError());
         need_eval1_ = (any_baro_ && !phys_) || any_ref_lj_;
         --n;
-        if (!tuned_) {
+        if (!tuned_ && !rule_bps_) {
             int used = 0;
             int rc = autotune(n, &used);
             if (rc) return rc;
@@ -1462,9 +1470,11 @@ int Batch::capture_steps(int n, cudaGraphExec_t* out) {
 }
 
 // Pair-kernel launch shape by measurement: each candidate runs kTuneSteps real
-// steps (eagerly, in the same order as the captured step) timed with events on
-// the main stream, which the bonded / PME stream joins every step; the fastest
-// median step wins and is cached for this kind of batch.  The candidates give
+// steps timed with events on the main stream, which the bonded / PME stream
+// joins every step; the fastest median step wins and is cached for this kind
+// of batch.  The steps are launched as one-step graphs, as the run launches
+// them: issued kernel by kernel, a step of a few ten microseconds was as long
+// as the host took to issue it and the choice was noise.  The candidates give
 // bit-identical results, so tuning steps are ordinary steps of the run.  Runs
 // only when the call has enough steps to spare.
 int Batch::autotune(int max_steps, int* used) {
@@ -1477,6 +1487,8 @@ int Batch::autotune(int max_steps, int* used) {
     std::vector<TuneChoice> cand;
     for (const TuneChoice& c : kTuneCand)
         if (c.form == form) cand.push_back(c);
+    for (TuneChoice& c : cand)
+        if (c.bps == nb_blocks_per_sm_) std::swap(c, cand[0]);
     const int n_cand = static_cast<int>(cand.size());
     if (max_steps < n_cand * kTuneSteps) return DMDGPU_OK;
     std::vector<cudaEvent_t> ev(kTuneSteps + 1);
@@ -1487,16 +1499,22 @@ int Batch::autotune(int max_steps, int* used) {
         nb_form_ = cand[c].form;
         nb_blocks_per_sm_ = cand[c].bps;
         std::vector<float> t(kTuneSteps);
+        cudaGraphExec_t ge = nullptr;
+        const long long before = launches_;
+        int rc = capture_steps(1, &ge);
+        if (rc) return rc;
+        launches_ = before + kTuneSteps * (launches_ - before);
         CK(cudaEventRecord(ev[0], stream_));
         for (int i = 0; i < kTuneSteps; ++i) {
-            enqueue_step();
+            CK(cudaGraphLaunch(ge, stream_));
             CK(cudaEventRecord(ev[i + 1], stream_));
         }
-        CK(cudaGetLastError());
         CK(cudaEventSynchronize(ev[kTuneSteps]));
+        cudaGraphExecDestroy(ge);
         for (int i = 0; i < kTuneSteps; ++i) CK(cudaEventElapsedTime(&t[i], ev[i], ev[i + 1]));
         std::sort(t.begin(), t.end());
-        const float med = t[kTuneSteps / 2];
+        // the shape the rule gave (timed first) stays unless another is clearly better
+        const float med = t[kTuneSteps / 2] * (c == 0 ? 0.97f : 1.0f);
         if (med < best_ms) {
             best_ms = med;
             best = cand[c];
@@ -1522,6 +1540,7 @@ int Batch::rebuild_in_frame(const std::vector<char>& sel) {
     const int R = static_cast<int>(order_.size());
     if (R == 0) return DMDGPU_OK;
     std::vector<RepState> cur(R), tmp(R);
+    n_chunks_built_.resize(R, 0);
     CK(cudaStreamSynchronize(stream_));
     CK(cudaMemcpy(cur.data(), d_st_, sizeof(RepState) * R, cudaMemcpyDeviceToHost));
     tmp = cur;
@@ -1547,6 +1566,7 @@ int Batch::rebuild_in_frame(const std::vector<char>& sel) {
             continue;
         }
         RepState& f = tmp[k];
+        n_chunks_built_[k] = f.n_chunks;
         f.L = cur[k].L;
         f.invL = cur[k].invL;
         f.L_build = cur[k].L_build;

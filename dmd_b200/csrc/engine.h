@@ -207,6 +207,8 @@ class Batch {
     void set_node_priorities(cudaGraph_t g);
     int nb_form_ = 1;           // pair-kernel form (NbForm; autotuned)
     bool tuned_ = false;
+    bool rule_bps_ = false;     // the launch shape follows from the table (no PME chain)
+    std::vector<int> n_chunks_built_;  // chunks per packed replica at its last build in frame
     long long launches_ = 0;
     long long per_step_launches_ = 0;
     long long used_bytes_ = 0;

@@ -60,6 +60,7 @@ __device__ __forceinline__ float erfc_as(float x, float e) {
 }
 
 __device__ __forceinline__ void flush_acc(const Dev& d, int r, Acc& acc) {
+    if (!__any_sync(FULL, (acc.lj | acc.c | acc.v) != 0)) return;  // no energies this evaluation
     long long lj = warp_sum_ll(acc.lj), c = warp_sum_ll(acc.c), v = warp_sum_ll(acc.v);
     if ((threadIdx.x & 31) == 0 && r >= 0) {
         if (lj) fix_add(&d.st[r].e_acc[E_LJ], lj);
@@ -137,7 +138,7 @@ __device__ __forceinline__ float pair_f(float r2, float c6f, float c12f, float q
 // evaluation, as the reference does (Cell::minimum_image, cell.cpp:26-38): in
 // such a box the nearest image of a listed pair can change between list
 // builds, so the image frozen at the build is not enough.
-template <bool PHYS, bool SAME, bool ENERGY, bool MI>
+template <bool PHYS, bool SAME, bool ENERGY, bool MI, bool ONE = false>
 __device__ __forceinline__ void nb_chunk(const Dev& d, const Rep& R, RepState* s, int c, int lane,
                                          ChunkStage& S, const float4* lj_tab, Acc& acc) {
     const double L = s->L;
@@ -189,15 +190,16 @@ __device__ __forceinline__ void nb_chunk(const Dev& d, const Rep& R, RepState* s
     uint32_t band = 0;
     const int src_lane = (lane + 1) & 31;
 #pragma unroll 1
-    for (int kk = 0; kk < 32; kk += 8) {
+    for (int kk = 0; kk < 32; kk += 4) {
         const float4* px = S.xq + lane + kk;
         const int* pt = S.tj + lane + kk;
         uint32_t b8 = 0;
+        float tmin = 1e30f;  // smallest |r^2 - rc^2| of the eight rounds
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < 4; ++u) {
             const bool bit = (rm >> u) & 1u;
             const float4 pj = px[u];
-            const float4 p = lj[pt[u]];
+            const float4 p = ONE ? lj[0] : lj[pt[u]];
             float dx = pj.x - xi.x, dy = pj.y - xi.y, dz = pj.z - xi.z;
             if (MI) {
                 dx = fmaf(-Lf, rintf(dx * iLf), dx);
@@ -208,10 +210,13 @@ __device__ __forceinline__ void nb_chunk(const Dev& d, const Rep& R, RepState* s
             if (!ENERGY && (!PHYS || SAME)) {
                 // one cutoff: evaluate with the table coefficients and keep the
                 // force only for interacting pairs (a masked self pair of a
-                // diagonal chunk gives a non-finite f, which the select drops)
-                const bool near = bit & (fabsf(d2 - rl2) < wl);
-                const bool in = bit & !near & (d2 < rl2);
-                b8 |= static_cast<uint32_t>(near) << u;
+                // diagonal chunk gives a non-finite f, which the select drops).
+                // Pairs in the cutoff band are left to the pass after the loop;
+                // which they are is found only when some round of the eight
+                // had one (two instructions per pair instead of five).
+                const float t = d2 - rl2;
+                tmin = fminf(tmin, fabsf(t));
+                const bool in = bit & (t <= -wl);
                 float ir6, rinv, erfc_ar;
                 const float fa = pair_f<PHYS>(d2, p.z, p.w, keqi * pj.w, alpha, a2l2e, c2a, ir6, rinv, erfc_ar);
                 const float f = in ? fa : 0.f;
@@ -259,8 +264,21 @@ __device__ __forceinline__ void nb_chunk(const Dev& d, const Rep& R, RepState* s
             fjy = __shfl_sync(FULL, fjy, src_lane);
             fjz = __shfl_sync(FULL, fjz, src_lane);
         }
+        if (!ENERGY && (!PHYS || SAME) && tmin < wl) {  // rare: which of the eight rounds
+            for (int u = 0; u < 4; ++u) {
+                const float4 pj = px[u];
+                float dx = pj.x - xi.x, dy = pj.y - xi.y, dz = pj.z - xi.z;
+                if (MI) {
+                    dx = fmaf(-Lf, rintf(dx * iLf), dx);
+                    dy = fmaf(-Lf, rintf(dy * iLf), dy);
+                    dz = fmaf(-Lf, rintf(dz * iLf), dz);
+                }
+                const float t = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) - rl2;
+                b8 |= static_cast<uint32_t>(((rm >> u) & 1u) & (fabsf(t) < wl)) << u;
+            }
+        }
         band |= b8 << kk;
-        rm >>= 8;
+        rm >>= 4;
     }
     // after 32 rounds lane l holds the forces of entry l again
     while (band) {  // pairs at a cutoff (rare): FP64 reference membership
@@ -340,13 +358,15 @@ __global__ void __launch_bounds__(256, PHYS ? 3 : 4) k_nb_f32(Dev d) {
     const int total = d.chunk_prefix[d.n_rep];
     Acc acc{0, 0, 0};
     int cur = -1;
-    // chunks are taken one per warp from a counter, so warps on SMs shared with
-    // the concurrent PME kernels simply take fewer
+    // A warp's first chunk is its own number (warp 0 of every block first, so a
+    // short list spreads over all SMs); the chunks after the first nw are taken
+    // one per warp from a counter, so warps on SMs shared with the concurrent
+    // PME kernels simply take fewer.  Claiming the first chunk from the counter
+    // too put one atomic per warp (4,736 of them) on one address, which alone
+    // took 5.3 us: 1,000 LJ atoms, 223 chunks, 8.9 -> 5.7 us per launch; decane 4k 10.1 -> 6.9 us.
     int* counter = MIK ? d.nb_work_mi : d.nb_work;
-    for (;;) {
-        int w = 0;
-        if (lane == 0) w = atomicAdd(counter, 1);
-        w = __shfl_sync(FULL, w, 0);
+    const int nw = gridDim.x * 8;
+    for (int w = blockIdx.x + gridDim.x * wib;;) {
         if (w >= total) break;
         const int r = chunk_replica(d.chunk_prefix, d.n_rep, w);
         if (r != cur) {
@@ -381,7 +401,13 @@ __global__ void __launch_bounds__(256, PHYS ? 3 : 4) k_nb_f32(Dev d) {
                     }
                 }
             }
-            if (lane == 0) atomicMax(counter, d.chunk_prefix[next]);
+            if (total <= nw) break;  // every chunk is some warp's first
+            if (lane == 0) {
+                const int skip = d.chunk_prefix[next] - nw;
+                if (skip > 0) atomicMax(counter, skip);
+                w = nw + atomicAdd(counter, 1);
+            }
+            w = __shfl_sync(FULL, w, 0);
             continue;
         }
         const int c = R.chunk_begin + (w - d.chunk_prefix[r]);
@@ -401,10 +427,15 @@ __global__ void __launch_bounds__(256, PHYS ? 3 : 4) k_nb_f32(Dev d) {
             else if (same) nb_chunk<true, true, true, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
             else nb_chunk<true, false, true, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
         } else {
-            if (!coul) nb_chunk<false, false, false, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
-            else if (same) nb_chunk<true, true, false, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
+            if (!coul) {
+                if (R.n_types == 1) nb_chunk<false, false, false, false, true>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
+                else nb_chunk<false, false, false, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
+            } else if (same) nb_chunk<true, true, false, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
             else nb_chunk<true, false, false, false>(d, R, s, c, lane, s_stage[wib], lj_tab, acc);
         }
+        if (total <= nw) break;  // every chunk is some warp's first
+        if (lane == 0) w = nw + atomicAdd(counter, 1);
+        w = __shfl_sync(FULL, w, 0);
     }
     flush_acc(d, cur, acc);
 }
