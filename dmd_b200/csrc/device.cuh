@@ -10,6 +10,14 @@ namespace dmd {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// Start of a kernel that launch_chained may have launched: wait until the
+// kernel before it has completed and its writes are visible, then let the next
+// one be set up.  No effect under an ordinary launch.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Cell::minimum_image, orthorhombic branch (src/core/cell.cpp:26-38), with the
 // reference's rounding: d - round(d * (1/L)) * L, no contraction.  CUDA's
 // round() rounds half away from zero like std::round.

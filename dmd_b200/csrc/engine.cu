@@ -1227,7 +1227,8 @@ void Batch::enqueue_eval(int pass) {
     // and energy sums are fixed-point atomics (order-free).  The pair kernel (the
     // longest branch, persistent) is issued first so its blocks take their SM
     // slots before the short PME and bonded blocks fill the rest.
-    cudaEventRecord(ev_fork_, stream_);
+    const bool bonded = d.n_bonds + d.n_angles + d.n_dih + d.n_imp + d.n_excl > 0;
+    if (any_pme_ || bonded) cudaEventRecord(ev_fork_, stream_);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (prof_nb_) {
         e0 = next_event();
@@ -1239,9 +1240,8 @@ void Batch::enqueue_eval(int pass) {
         record(e1, stream_);
         prof_nb_->emplace_back(e0, e1);
     }
-    cudaStreamWaitEvent(aux_stream_, ev_fork_, 0);
-    cudaStreamWaitEvent(bond_stream_, ev_fork_, 0);
     if (any_pme_) {
+        cudaStreamWaitEvent(aux_stream_, ev_fork_, 0);
         if (prof_pme_) {
             e0 = next_event();
             record(e0, aux_stream_);
@@ -1280,11 +1280,17 @@ void Batch::enqueue_eval(int pass) {
             prof_pme_->emplace_back(e0, e1);
         }
     }
-    cudaEventRecord(ev_join_, aux_stream_);
-    launch_bonded(d, fp64_, phys_, bond_stream_, &launches_);
-    cudaEventRecord(ev_join_b_, bond_stream_);
-    cudaStreamWaitEvent(stream_, ev_join_, 0);
-    cudaStreamWaitEvent(stream_, ev_join_b_, 0);
+    if (bonded) {
+        cudaStreamWaitEvent(bond_stream_, ev_fork_, 0);
+        launch_bonded(d, fp64_, phys_, bond_stream_, &launches_);
+        cudaEventRecord(ev_join_b_, bond_stream_);
+        cudaStreamWaitEvent(stream_, ev_join_b_, 0);
+    }
+    if (any_pme_) {
+        cudaEventRecord(ev_join_, aux_stream_);
+        cudaStreamWaitEvent(stream_, ev_join_, 0);
+    }
+    joined_ = bonded || any_pme_;
     // the second pass of a step is closed by k_replica_update
     if (pass != PASS_SECOND) launch_eval_end(d, stream_, &launches_);
 }
@@ -1301,7 +1307,7 @@ void Batch::enqueue_step() {
     launch_kick_drift(dev_, fp64_, stream_, &launches_);
     if (any_cons_) launch_shake(dev_, stream_, &launches_);
     enqueue_eval(PASS_SECOND);
-    launch_kick2(dev_, any_andersen_ref_, any_andersen_phys_, stream_, &launches_);
+    launch_kick2(dev_, any_andersen_ref_, any_andersen_phys_, !joined_, stream_, &launches_);
     if (any_cons_) launch_rattle(dev_, stream_, &launches_);
     launch_replica_update(dev_, stream_, &launches_);
     if (any_baro_ && !phys_) launch_apply_scale(dev_, fp64_, stream_, &launches_);

@@ -192,6 +192,7 @@ class Batch {
     std::map<int, std::pair<cufftHandle, cufftHandle>> plans_;
     cudaGraphExec_t graph_ = nullptr;       // one step
     cudaGraphExec_t graph_many_ = nullptr;  // kManySteps steps (tables that keep running)
+    bool joined_ = false;                   // the last evaluation joined other streams
     long long steps_run_ = 0;               // steps launched from graph_ or graph_many_
     int capture_steps(int n, cudaGraphExec_t* out);
     void drop_graphs();

@@ -286,6 +286,7 @@ __device__ __forceinline__ bool mesh_coord(double x, double invL, int K, int& m0
 // the fixed-point mesh on its own; the integer sums do not depend on order.
 template <typename T>
 __global__ void k_pme_spread(Dev d) {
+    chain_wait();
     const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int a = static_cast<int>(t >> 4);
     if (a >= d.n_atoms) return;
@@ -330,6 +331,7 @@ __global__ void k_pme_spread(Dev d) {
 // per-replica test delays the loads.
 template <typename T>
 __global__ void k_pme_convert(Dev d) {
+    chain_wait();
     const int r = d.conv_block_rep[blockIdx.x];
     const Rep& R = d.rep[r];
     const int loc0 = 1024 * (blockIdx.x - R.conv_block_begin) + 4 * threadIdx.x;
@@ -378,6 +380,7 @@ __global__ void k_pme_convert(Dev d) {
 // energies are read.
 template <typename T>
 __global__ void k_pme_influence(Dev d) {
+    chain_wait();
     const int r = d.pme_block_rep[blockIdx.x];
     const Rep& R = d.rep[r];
     RepState* s = d.st + r;
@@ -455,6 +458,7 @@ __global__ void k_pme_influence(Dev d) {
 // order.  The x and y weights are computed once per thread.
 template <typename T>
 __global__ void k_pme_gather(Dev d) {
+    chain_wait();
     const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int a = static_cast<int>(t >> 2);
     // every condition below is uniform over the atom's 4 lanes
@@ -575,21 +579,21 @@ void launch_pme_spread(const Dev& d, bool fp64, cudaStream_t st, long long* nlau
 
 void launch_pme_convert(const Dev& d, bool fp64, int n_blocks, cudaStream_t st, long long* nlaunch) {
     if (n_blocks <= 0) return;
-    if (fp64) k_pme_convert<double><<<n_blocks, 256, 0, st>>>(d);
-    else k_pme_convert<float><<<n_blocks, 256, 0, st>>>(d);
+    if (fp64) launch_chained(k_pme_convert<double>, n_blocks, 256, st, d);
+    else launch_chained(k_pme_convert<float>, n_blocks, 256, st, d);
     ++*nlaunch;
 }
 
 void launch_pme_influence(const Dev& d, bool fp64, int n_blocks, cudaStream_t st, long long* nlaunch) {
-    if (fp64) k_pme_influence<double><<<n_blocks, 256, 0, st>>>(d);
-    else k_pme_influence<float><<<n_blocks, 256, 0, st>>>(d);
+    if (fp64) launch_chained(k_pme_influence<double>, n_blocks, 256, st, d);
+    else launch_chained(k_pme_influence<float>, n_blocks, 256, st, d);
     ++*nlaunch;
 }
 
 void launch_pme_gather(const Dev& d, bool fp64, cudaStream_t st, long long* nlaunch) {
     const int T = 256, g = static_cast<int>((4LL * d.n_atoms + T - 1) / T);
-    if (fp64) k_pme_gather<double><<<g, T, 0, st>>>(d);
-    else k_pme_gather<float><<<g, T, 0, st>>>(d);
+    if (fp64) launch_chained(k_pme_gather<double>, g, T, st, d);
+    else launch_chained(k_pme_gather<float>, g, T, st, d);
     ++*nlaunch;
 }
 

@@ -31,6 +31,7 @@ namespace dmd {
 namespace {
 
 __global__ void k_eval_begin(Dev d, int pass) {
+    chain_wait();
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r == 0) {
         *d.nb_work = 0;
@@ -84,6 +85,7 @@ __global__ void k_eval_begin(Dev d, int pass) {
 }
 
 __global__ void k_eval_end(Dev d) {
+    chain_wait();
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= d.n_rep) return;
     RepState* s = d.st + r;
@@ -95,6 +97,7 @@ __global__ void k_eval_end(Dev d) {
 }
 
 __global__ void k_clear_forces(Dev d) {
+    chain_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < d.n_slots) {
         int r = d.tile_rep[i >> 5];
@@ -142,6 +145,7 @@ __device__ __forceinline__ void skin_check(const Dev& d, RepState* s, const Rep&
 // forces are read and written coalesced; only the pair forces and the mirror
 // are addressed through the atom's slot.
 __global__ void k_kick_drift(Dev d) {
+    chain_wait();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= d.n_atoms) return;
     const int r = d.atom_rep[a];
@@ -197,6 +201,7 @@ __device__ __forceinline__ void philox(uint32_t c[4], uint32_t k0, uint32_t k1) 
 
 // Second half kick, optional Andersen collisions, per-tile KE and r.F partials.
 __global__ void k_kick2(Dev d, int andersen_ref, int andersen_phys) {
+    chain_wait();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int t = slot >> 5;
@@ -369,6 +374,7 @@ __device__ __forceinline__ void rattle_triangle(const double (&x)[3], const doub
 // pending barostat scale), and SHAKE's displacement is also given to the
 // half-step velocities (v += dx / dt).
 __global__ void k_shake(Dev d) {
+    chain_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= d.n_cgroups) return;
     const int r = d.cgroup_rep[g];
@@ -457,6 +463,7 @@ __global__ void k_shake(Dev d) {
 // Constraints::apply_rattle (constraints.cpp:49-91), after the second half
 // kick: the same group sweeps on r.v, lambda = r.v / (r^2 (1/m_i + 1/m_j)).
 __global__ void k_rattle(Dev d) {
+    chain_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= d.n_cgroups) return;
     const int r = d.cgroup_rep[g];
@@ -520,6 +527,7 @@ __global__ void k_rattle(Dev d) {
 // Per-tile kinetic-energy partials again after RATTLE (the thermostat reads the
 // constrained velocities; same expression and order as k_kick2's).
 __global__ void k_tile_ke(Dev d) {
+    chain_wait();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int t = slot >> 5;
@@ -598,6 +606,7 @@ __device__ void block_sum4(double v[4], double (*sh)[4]) {
 // (berendsen_barostat.cpp:14-66); one block per replica.  Tile partials of KE
 // and r.F and the PME blocks' energy / virial partials are summed together.
 __global__ void k_replica_update(Dev d) {
+    chain_wait();
     __shared__ double sh[8][4];
     const int r = blockIdx.x;
     RepState* s = d.st + r;
@@ -689,6 +698,7 @@ __global__ void k_replica_update(Dev d) {
 
 // BerendsenBarostat position scaling (berendsen_barostat.cpp:60-65).
 __global__ void k_apply_scale(Dev d) {
+    chain_wait();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= d.n_slots) return;
     const int r = d.tile_rep[slot >> 5];
@@ -757,41 +767,43 @@ __global__ void k_write_mirror(Dev d) {
 }  // namespace
 
 void launch_eval_begin(const Dev& d, int pass, cudaStream_t st, long long* n) {
-    k_eval_begin<<<(d.n_rep + 127) / 128, 128, 0, st>>>(d, pass);
+    launch_chained(k_eval_begin, (d.n_rep + 127) / 128, 128, st, d, pass);
     ++*n;
 }
 void launch_clear_forces(const Dev& d, cudaStream_t st, long long* n) {
     const int m = d.n_slots > d.n_atoms ? d.n_slots : d.n_atoms;
-    k_clear_forces<<<(m + 255) / 256, 256, 0, st>>>(d);
+    launch_chained(k_clear_forces, (m + 255) / 256, 256, st, d);
     ++*n;
 }
 void launch_eval_end(const Dev& d, cudaStream_t st, long long* n) {
-    k_eval_end<<<(d.n_rep + 127) / 128, 128, 0, st>>>(d);
+    launch_chained(k_eval_end, (d.n_rep + 127) / 128, 128, st, d);
     ++*n;
 }
 void launch_kick_drift(const Dev& d, bool, cudaStream_t st, long long* n) {
-    k_kick_drift<<<(d.n_atoms + 255) / 256, 256, 0, st>>>(d);
+    launch_chained(k_kick_drift, (d.n_atoms + 255) / 256, 256, st, d);
     ++*n;
 }
-void launch_kick2(const Dev& d, bool andersen_ref, bool andersen_phys, cudaStream_t st, long long* n) {
-    k_kick2<<<(d.n_slots + 255) / 256, 256, 0, st>>>(d, andersen_ref ? 1 : 0, andersen_phys ? 1 : 0);
+void launch_kick2(const Dev& d, bool andersen_ref, bool andersen_phys, bool chained, cudaStream_t st, long long* n) {
+    const int g = (d.n_slots + 255) / 256, ar = andersen_ref ? 1 : 0, ap = andersen_phys ? 1 : 0;
+    if (chained) launch_chained(k_kick2, g, 256, st, d, ar, ap);
+    else k_kick2<<<g, 256, 0, st>>>(d, ar, ap);
     ++*n;
 }
 void launch_shake(const Dev& d, cudaStream_t st, long long* n) {
-    k_shake<<<(d.n_cgroups + 63) / 64, 64, 0, st>>>(d);
+    launch_chained(k_shake, (d.n_cgroups + 63) / 64, 64, st, d);
     ++*n;
 }
 void launch_rattle(const Dev& d, cudaStream_t st, long long* n) {
-    k_rattle<<<(d.n_cgroups + 63) / 64, 64, 0, st>>>(d);
-    k_tile_ke<<<(d.n_slots + 255) / 256, 256, 0, st>>>(d);
+    launch_chained(k_rattle, (d.n_cgroups + 63) / 64, 64, st, d);
+    launch_chained(k_tile_ke, (d.n_slots + 255) / 256, 256, st, d);
     *n += 2;
 }
 void launch_replica_update(const Dev& d, cudaStream_t st, long long* n) {
-    k_replica_update<<<d.n_rep, 256, 0, st>>>(d);
+    launch_chained(k_replica_update, d.n_rep, 256, st, d);
     ++*n;
 }
 void launch_apply_scale(const Dev& d, bool, cudaStream_t st, long long* n) {
-    k_apply_scale<<<(d.n_slots + 255) / 256, 256, 0, st>>>(d);
+    launch_chained(k_apply_scale, (d.n_slots + 255) / 256, 256, st, d);
     ++*n;
 }
 void launch_finalize_velocities(const Dev& d, cudaStream_t st, long long* n) {

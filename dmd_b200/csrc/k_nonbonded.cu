@@ -347,6 +347,7 @@ constexpr int LJ_SMEM = 512;
 // tables without real-space Coulomb) fits 64 (4 blocks per SM).
 template <bool PHYS, bool LJS, bool MIK>
 __global__ void __launch_bounds__(256, PHYS ? 3 : 4) k_nb_f32(Dev d) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     __shared__ ChunkStage s_stage[8];
@@ -637,6 +638,7 @@ __device__ __forceinline__ void nb_cluster(const Dev& d, const Rep& R, RepState*
 // (up to 128 registers per thread: 2 blocks of 256 threads per SM).
 template <bool PHYS, bool LJS>
 __global__ void __launch_bounds__(256, 2) k_nb8_f32(Dev d) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     __shared__ ClusterStage s_stage[8];
@@ -682,6 +684,7 @@ __global__ void __launch_bounds__(256, 2) k_nb8_f32(Dev d) {
 
 template <bool PHYS>
 __global__ void __launch_bounds__(256) k_nb_f64(Dev d) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     __shared__ double4 s_xj[8][32];
@@ -824,8 +827,8 @@ void configure_nonbonded_kernels() {
 void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_per_sm, int form,
                       cudaStream_t st, long long* nlaunch) {
     if (fp64) {
-        if (phys) k_nb_f64<true><<<n_sm * 8, 256, 0, st>>>(d);
-        else k_nb_f64<false><<<n_sm * 8, 256, 0, st>>>(d);
+        if (phys) launch_chained(k_nb_f64<true>, n_sm * 8, 256, st, d);
+        else launch_chained(k_nb_f64<false>, n_sm * 8, 256, st, d);
     } else {
         const bool ljs = d.n_lj <= LJ_SMEM;
         // a table without real-space Coulomb runs the LJ-only instantiation
@@ -839,30 +842,30 @@ void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_p
         if (form == NB_CLUSTER8 && d.cl_j) {
             const int g = n_sm * std::min(bps, 2);
             if (phys) {
-                if (ljs) k_nb8_f32<true, true><<<g, 256, 0, st>>>(d);
-                else k_nb8_f32<true, false><<<g, 256, 0, st>>>(d);
+                if (ljs) launch_chained(k_nb8_f32<true, true>, g, 256, st, d);
+                else launch_chained(k_nb8_f32<true, false>, g, 256, st, d);
             } else {
-                if (ljs) k_nb8_f32<false, true><<<g, 256, 0, st>>>(d);
-                else k_nb8_f32<false, false><<<g, 256, 0, st>>>(d);
+                if (ljs) launch_chained(k_nb8_f32<false, true>, g, 256, st, d);
+                else launch_chained(k_nb8_f32<false, false>, g, 256, st, d);
             }
         } else {
             const int g = n_sm * std::min(bps, max_bps);
             if (phys) {
-                if (ljs) k_nb_f32<true, true, false><<<g, 256, 0, st>>>(d);
-                else k_nb_f32<true, false, false><<<g, 256, 0, st>>>(d);
+                if (ljs) launch_chained(k_nb_f32<true, true, false>, g, 256, st, d);
+                else launch_chained(k_nb_f32<true, false, false>, g, 256, st, d);
             } else {
-                if (ljs) k_nb_f32<false, true, false><<<g, 256, 0, st>>>(d);
-                else k_nb_f32<false, false, false><<<g, 256, 0, st>>>(d);
+                if (ljs) launch_chained(k_nb_f32<false, true, false>, g, 256, st, d);
+                else launch_chained(k_nb_f32<false, false, false>, g, 256, st, d);
             }
         }
         if (d.mi_split) {  // narrow-box replicas: their own kernel on the same stream
             const int g = n_sm * std::min(bps, max_bps);
             if (phys) {
-                if (ljs) k_nb_f32<true, true, true><<<g, 256, 0, st>>>(d);
-                else k_nb_f32<true, false, true><<<g, 256, 0, st>>>(d);
+                if (ljs) launch_chained(k_nb_f32<true, true, true>, g, 256, st, d);
+                else launch_chained(k_nb_f32<true, false, true>, g, 256, st, d);
             } else {
-                if (ljs) k_nb_f32<false, true, true><<<g, 256, 0, st>>>(d);
-                else k_nb_f32<false, false, true><<<g, 256, 0, st>>>(d);
+                if (ljs) launch_chained(k_nb_f32<false, true, true>, g, 256, st, d);
+                else launch_chained(k_nb_f32<false, false, true>, g, 256, st, d);
             }
             *nlaunch += 1;
         }
