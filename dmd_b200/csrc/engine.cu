@@ -1217,8 +1217,11 @@ int Batch::pack() {
 // ---------------------------------------------------------------------------
 void Batch::enqueue_eval(int pass) {
     Dev& d = dev_;
-    launch_eval_begin(d, pass, stream_, &launches_);
-    if (pass != PASS_SECOND) launch_clear_forces(d, stream_, &launches_);
+    // (the second pass of a step begins before its drift)
+    if (pass != PASS_SECOND) {
+        launch_eval_begin(d, pass, stream_, &launches_);
+        launch_clear_forces(d, stream_, &launches_);
+    }
     // The list rebuild (a cooperative launch: it needs the whole GPU) goes first;
     // it returns at once on steps without a rebuild.
     enqueue_rebuild();
@@ -1299,17 +1302,20 @@ void Batch::enqueue_eval(int pass) {
 // some replica's rebuild flag is set.
 void Batch::enqueue_rebuild() { launch_rebuild(dev_, d_bin_rep_, n_sm_, stream_, &launches_); }
 
-void Batch::enqueue_step() {
+// begun: the step before it in the same launch began this one; next: another
+// step follows in the same launch and this one begins it (k_replica_update).
+void Batch::enqueue_step(bool begun, bool next) {
     // The first evaluation repeats the previous step's second one unless the
     // barostat moved the atoms, the REF list cadence rebuilds now, or no forces
     // exist yet; only then is it issued (its kernels skip replicas that do not need it).
     if (need_eval1_) enqueue_eval(PASS_FIRST);
+    if (!begun) launch_eval_begin(dev_, PASS_SECOND, stream_, &launches_);
     launch_kick_drift(dev_, fp64_, stream_, &launches_);
     if (any_cons_) launch_shake(dev_, stream_, &launches_);
     enqueue_eval(PASS_SECOND);
     launch_kick2(dev_, any_andersen_ref_, any_andersen_phys_, !joined_, stream_, &launches_);
     if (any_cons_) launch_rattle(dev_, stream_, &launches_);
-    launch_replica_update(dev_, stream_, &launches_);
+    launch_replica_update(dev_, next, stream_, &launches_);
     if (any_baro_ && !phys_) launch_apply_scale(dev_, fp64_, stream_, &launches_);
 }
 
@@ -1466,7 +1472,9 @@ int Batch::run_steps(int n) {
 int Batch::capture_steps(int n, cudaGraphExec_t* out) {
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < n; ++k) enqueue_step();
+    // a first evaluation or the REF barostat's scaling comes between two steps
+    const bool between = need_eval1_ || (any_baro_ && !phys_);
+    for (int k = 0; k < n; ++k) enqueue_step(k > 0 && !between, k + 1 < n && !between);
     CK(cudaStreamEndCapture(stream_, &g));
     set_node_priorities(g);
     const cudaError_t e = cudaGraphInstantiate(out, g, cudaGraphInstantiateFlagUseNodePriority);

@@ -150,7 +150,7 @@ class Batch {
     int build_host(HostRep& hr, unsigned comp_mask);
     void enqueue_eval(int pass);
     void enqueue_rebuild();
-    void enqueue_step();
+    void enqueue_step(bool begun = false, bool next = false);
     int run_steps(int n);
     int autotune(int max_steps, int* used);
     int rebuild_in_frame(const std::vector<char>& sel);

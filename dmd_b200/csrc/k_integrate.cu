@@ -30,58 +30,78 @@ namespace dmd {
 
 namespace {
 
+// Work counters and the rebuild's grid barrier, before an evaluation.
+__device__ __forceinline__ void reset_counters(const Dev& d) {
+    *d.nb_work = 0;
+    if (d.nb_work_mi) *d.nb_work_mi = 0;
+    d.grid_bar[0] = 0;  // arrivals (the generation word keeps counting)
+}
+
+// A force evaluation of replica r (ev) is about to start.
+__device__ __forceinline__ void begin_eval(RepState& s, const Rep& R, bool ev, bool want_e) {
+    s.eval = ev;
+    s.green_ok = (s.green_L == s.L) ? 1 : 0;
+    s.want_e = want_e;
+    if (ev) {
+        for (int k = 0; k < N_EACC; ++k) s.e_acc[k] = 0;
+        s.e_recip = 0.0;
+        s.vir_recip = 0.0;
+        if (!(R.flags & F_PHYS) && (R.flags & F_LJ) && s.lj_counter >= 10) s.rebuild = 1;
+    }
+}
+
+// Start of a step, before its kick and drift: which replicas advance, the
+// pending scales handed to k_kick_drift, the box that follows the positions it
+// scales, and the step's (second) evaluation.  Runs in k_eval_begin ahead of
+// the first step of a launch, and at the end of k_replica_update between the
+// steps of one launch.
+__device__ __forceinline__ void begin_step(RepState& s, const Rep& R) {
+    s.active = (s.step < s.target_step) ? 1 : 0;
+    s.dr_move = s.active;
+    s.dr_vscale = s.vscale;
+    s.dr_pscale = s.pscale;
+    s.dr_L = s.L;
+    // a replica that has reached its target keeps its pending thermostat scale
+    // for the next read of its velocities
+    if (s.active) s.vscale = 1.0;
+    if (s.active && (R.flags & F_PHYS) && s.pscale != 1.0) {
+        s.L *= s.pscale;
+        s.invL = 1.0 / s.L;
+        s.pscale = 1.0;
+    }
+    // Pair energies and the pair virial are needed by single-point evaluations,
+    // by the evaluation that ends a run (its energies are what the host reads) and,
+    // with the PHYS barostat, every step (its pressure uses the atomic virial).
+    begin_eval(s, R, s.active, s.step + 1 >= s.target_step || ((R.flags & F_PHYS) && R.barostat));
+}
+
 __global__ void k_eval_begin(Dev d, int pass) {
     chain_wait();
     int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) {
-        *d.nb_work = 0;
-        if (d.nb_work_mi) *d.nb_work_mi = 0;
-        d.grid_bar[0] = 0;  // arrivals (the generation word keeps counting)
-    }
+    if (r == 0) reset_counters(d);
     if (r >= d.n_rep) return;
     RepState* s = d.st + r;
     const Rep& R = d.rep[r];
-    const bool ref_lj = !(R.flags & F_PHYS) && (R.flags & F_LJ);
-    // which replicas advance this step (the host may have moved the targets)
-    if (pass != PASS_SINGLE) s->active = (s->step < s->target_step) ? 1 : 0;
-    // REF: the barostat scale of the previous step has been applied; PHYS keeps
-    // its pending scale for k_kick_drift (positions) and the second pass (box),
-    // so an evaluation before the drift sees the unscaled pair.
-    if (pass == PASS_FIRST && !(R.flags & F_PHYS)) s->pscale = 1.0;
-    int ev;
+    if (pass == PASS_SECOND) {
+        begin_step(*s, R);
+        return;
+    }
+    bool ev = true;
     if (pass == PASS_FIRST) {
+        const bool ref_lj = !(R.flags & F_PHYS) && (R.flags & F_LJ);
+        // which replicas advance this step (the host may have moved the targets)
+        s->active = (s->step < s->target_step) ? 1 : 0;
+        // REF: the barostat scale of the previous step has been applied; PHYS keeps
+        // its pending scale for the drift, so an evaluation before it sees the
+        // unscaled pair.
+        if (!(R.flags & F_PHYS)) s->pscale = 1.0;
         ev = s->active && ((R.barostat != 0 && !(R.flags & F_PHYS)) || !s->have_forces ||
                            (ref_lj && s->lj_counter >= 10));
         // LennardJones::compute advances its counter on every call (lennard_jones.cpp:91)
         if (s->active && !ev && ref_lj) s->lj_counter += 1;
-    } else if (pass == PASS_SECOND) {
-        ev = s->active;
-        // consumed by k_kick_drift; a replica that has reached its target keeps
-        // its pending thermostat scale for the next read of its velocities
-        if (s->active) s->vscale = 1.0;
-        if (s->active && (R.flags & F_PHYS) && s->pscale != 1.0) {
-            // the box follows the positions k_kick_drift has just scaled
-            s->L *= s->pscale;
-            s->invL = 1.0 / s->L;
-            s->pscale = 1.0;
-        }
-    } else {
-        ev = 1;
     }
-    s->eval = ev;
-    s->green_ok = (s->green_L == s->L) ? 1 : 0;
-    // Pair energies and the pair virial are needed by single-point evaluations,
-    // by the evaluation that ends a run (its energies are what the host reads) and,
-    // with the PHYS barostat, every step (its pressure uses the atomic virial).
-    // Eval #1 never needs them: eval #2 of the same step overwrites its sums.
-    s->want_e = (pass == PASS_SINGLE) ||
-                (pass == PASS_SECOND && (s->step + 1 >= s->target_step || ((R.flags & F_PHYS) && R.barostat)));
-    if (ev) {
-        for (int k = 0; k < N_EACC; ++k) s->e_acc[k] = 0;
-        s->e_recip = 0.0;
-        s->vir_recip = 0.0;
-        if (ref_lj && s->lj_counter >= 10) s->rebuild = 1;
-    }
+    // eval #1 never needs energies: eval #2 of the same step overwrites its sums
+    begin_eval(*s, R, ev, pass == PASS_SINGLE);
 }
 
 __global__ void k_eval_end(Dev d) {
@@ -140,33 +160,48 @@ __device__ __forceinline__ void skin_check(const Dev& d, RepState* s, const Rep&
 // thermostat scale of the previous step applied first.  PHYS with a barostat:
 // the pending position scale s (1 otherwise, an exact multiply) is applied
 // before the drift, x <- s x + v dt, and the mirror is written for the box
-// s L that k_eval_begin stores next.
+// s L that begin_step has stored.
 // One thread per atom in reference order: the FP64 state, masses and bonded
 // forces are read and written coalesced; only the pair forces and the mirror
 // are addressed through the atom's slot.
+// The kernel before it (k_eval_begin or k_replica_update) writes replica state
+// only, so a chained launch loads everything else before it waits for that
+// kernel.  With k_kick2 and k_replica_update loading ahead the same way and the
+// next step begun by k_replica_update, a step of 1,000 LJ atoms takes 13.5 us
+// (18.8 with each kernel loading after its wait and k_eval_begin every step).
 __global__ void k_kick_drift(Dev d) {
-    chain_wait();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= d.n_atoms) return;
-    const int r = d.atom_rep[a];
+    const bool in = a < d.n_atoms;
+    int r = 0, slot = 0;
+    double inv_mass = 0, fx = 0, fy = 0, fz = 0, vx = 0, vy = 0, vz = 0, x = 0, y = 0, z = 0;
+    if (in) {
+        r = d.atom_rep[a];
+        slot = d.slot_of_atom[a];
+        inv_mass = 1.0 / d.mass[a];
+        fx = from_fix(d.fnx[slot] + d.fbx[a], FSCALE);
+        fy = from_fix(d.fny[slot] + d.fby[a], FSCALE);
+        fz = from_fix(d.fnz[slot] + d.fbz[a], FSCALE);
+        vx = d.vx[a];
+        vy = d.vy[a];
+        vz = d.vz[a];
+        x = d.x[a];
+        y = d.y[a];
+        z = d.z[a];
+    }
+    chain_wait();
+    if (!in) return;
     RepState* s = d.st + r;
-    if (!(s->step < s->target_step)) return;  // runs before this step's k_eval_begin
-    const int slot = d.slot_of_atom[a];
+    if (!s->dr_move) return;
     const Rep& R = d.rep[r];
     const double dt = R.dt, half_dt = 0.5 * dt;
-    const double inv_mass = 1.0 / d.mass[a];
-    const double lam = s->vscale;
-    const double fx = from_fix(d.fnx[slot] + d.fbx[a], FSCALE);
-    const double fy = from_fix(d.fny[slot] + d.fby[a], FSCALE);
-    const double fz = from_fix(d.fnz[slot] + d.fbz[a], FSCALE);
-    double vx = __dmul_rn(d.vx[a], lam), vy = __dmul_rn(d.vy[a], lam), vz = __dmul_rn(d.vz[a], lam);
-    vx = __dadd_rn(vx, __dmul_rn(__dmul_rn(fx, inv_mass), half_dt));
-    vy = __dadd_rn(vy, __dmul_rn(__dmul_rn(fy, inv_mass), half_dt));
-    vz = __dadd_rn(vz, __dmul_rn(__dmul_rn(fz, inv_mass), half_dt));
-    const double sc = s->pscale;
-    const double x = __dadd_rn(__dmul_rn(d.x[a], sc), __dmul_rn(vx, dt));
-    const double y = __dadd_rn(__dmul_rn(d.y[a], sc), __dmul_rn(vy, dt));
-    const double z = __dadd_rn(__dmul_rn(d.z[a], sc), __dmul_rn(vz, dt));
+    const double lam = s->dr_vscale;
+    vx = __dadd_rn(__dmul_rn(vx, lam), __dmul_rn(__dmul_rn(fx, inv_mass), half_dt));
+    vy = __dadd_rn(__dmul_rn(vy, lam), __dmul_rn(__dmul_rn(fy, inv_mass), half_dt));
+    vz = __dadd_rn(__dmul_rn(vz, lam), __dmul_rn(__dmul_rn(fz, inv_mass), half_dt));
+    const double sc = s->dr_pscale;
+    x = __dadd_rn(__dmul_rn(x, sc), __dmul_rn(vx, dt));
+    y = __dadd_rn(__dmul_rn(y, sc), __dmul_rn(vy, dt));
+    z = __dadd_rn(__dmul_rn(z, sc), __dmul_rn(vz, dt));
     d.vx[a] = vx;
     d.vy[a] = vy;
     d.vz[a] = vz;
@@ -179,7 +214,7 @@ __global__ void k_kick_drift(Dev d) {
     d.fbx[a] = 0;
     d.fby[a] = 0;
     d.fbz[a] = 0;
-    write_mirror(d, slot, a, x, y, z, s->L * sc);
+    write_mirror(d, slot, a, x, y, z, s->dr_L * sc);
     skin_check(d, s, R, a, x, y, z);
 }
 
@@ -200,27 +235,39 @@ __device__ __forceinline__ void philox(uint32_t c[4], uint32_t k0, uint32_t k1) 
 }
 
 // Second half kick, optional Andersen collisions, per-tile KE and r.F partials.
+// Only the forces come from the kernel before it in a chained launch: the rest
+// is loaded before the wait.
 __global__ void k_kick2(Dev d, int andersen_ref, int andersen_phys) {
-    chain_wait();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int t = slot >> 5;
     const int r = (t < d.n_tiles) ? d.tile_rep[t] : 0;
     RepState* s = d.st + r;
+    const Rep& R = d.rep[r];
     double ke = 0.0, w = 0.0;
-    if (slot < d.n_slots && s->active) {
-        const int a = d.atom_of_slot[slot];
+    int a = -1;
+    double m = 1, inv_mass = 1, vx = 0, vy = 0, vz = 0, x = 0, y = 0, z = 0;
+    if (slot < d.n_slots && s->active) a = d.atom_of_slot[slot];
+    if (a >= 0) {
+        m = d.mass[a];
+        inv_mass = 1.0 / m;
+        vx = d.vx[a];
+        vy = d.vy[a];
+        vz = d.vz[a];
+        x = d.x[a];
+        y = d.y[a];
+        z = d.z[a];
+    }
+    chain_wait();
+    {
         if (a >= 0) {
-            const Rep& R = d.rep[r];
             const double half_dt = 0.5 * R.dt;
-            const double m = d.mass[a];
-            const double inv_mass = 1.0 / m;
             const double fx = from_fix(d.fnx[slot] + d.fbx[a], FSCALE);
             const double fy = from_fix(d.fny[slot] + d.fby[a], FSCALE);
             const double fz = from_fix(d.fnz[slot] + d.fbz[a], FSCALE);
-            double vx = __dadd_rn(d.vx[a], __dmul_rn(__dmul_rn(fx, inv_mass), half_dt));
-            double vy = __dadd_rn(d.vy[a], __dmul_rn(__dmul_rn(fy, inv_mass), half_dt));
-            double vz = __dadd_rn(d.vz[a], __dmul_rn(__dmul_rn(fz, inv_mass), half_dt));
+            vx = __dadd_rn(vx, __dmul_rn(__dmul_rn(fx, inv_mass), half_dt));
+            vy = __dadd_rn(vy, __dmul_rn(__dmul_rn(fy, inv_mass), half_dt));
+            vz = __dadd_rn(vz, __dmul_rn(__dmul_rn(fz, inv_mass), half_dt));
             if (R.thermostat == 3 && R.t_freq * R.dt > 0.0) {
                 if (andersen_ref && d.and_flag && d.and_flag[a]) {
                     vx = d.and_v[3 * a];
@@ -254,7 +301,7 @@ __global__ void k_kick2(Dev d, int andersen_ref, int andersen_phys) {
             // kinetic_energy (thermostat.cpp:6-15) and virial (barostat.cpp:6-14) terms
             ke = __dmul_rn(__dmul_rn(0.5, m),
                            __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz)));
-            w = __dadd_rn(__dadd_rn(__dmul_rn(d.x[a], fx), __dmul_rn(d.y[a], fy)), __dmul_rn(d.z[a], fz));
+            w = __dadd_rn(__dadd_rn(__dmul_rn(x, fx), __dmul_rn(y, fy)), __dmul_rn(z, fz));
         }
     }
     ke = warp_sum_d(ke);
@@ -379,10 +426,10 @@ __global__ void k_shake(Dev d) {
     if (g >= d.n_cgroups) return;
     const int r = d.cgroup_rep[g];
     RepState* s = d.st + r;
-    if (!(s->step < s->target_step)) return;  // the replicas k_kick_drift moved
+    if (!s->dr_move) return;  // the replicas k_kick_drift moved
     const Rep& R = d.rep[r];
     const bool phys = (R.flags & F_PHYS) != 0;
-    const double L = phys ? s->L * s->pscale : s->L, inv = 1.0 / L, tol = R.cons_tol;
+    const double L = phys ? s->dr_L * s->dr_pscale : s->dr_L, inv = 1.0 / L, tol = R.cons_tol;
     const int c0 = d.cgroup_begin[g], c1 = d.cgroup_begin[g + 1];
     const int q0 = d.cgroup_atom_begin[g], q1 = d.cgroup_atom_begin[g + 1];
     const int na = d.n_atoms;
@@ -605,31 +652,41 @@ __device__ void block_sum4(double v[4], double (*sh)[4]) {
 // Thermostat (berendsen.cpp:13-28, nose_hoover.cpp:6-32) and Berendsen barostat
 // (berendsen_barostat.cpp:14-66); one block per replica.  Tile partials of KE
 // and r.F and the PME blocks' energy / virial partials are summed together.
-__global__ void k_replica_update(Dev d) {
-    chain_wait();
+// With `next` the next step of the same launch begins here too (begin_step).
+// In a chained launch only the tile partials come from the kernel before it:
+// the replica's records and the PME partials are loaded before the wait.
+__global__ void k_replica_update(Dev d, int next) {
     __shared__ double sh[8][4];
     const int r = blockIdx.x;
     RepState* s = d.st + r;
-    if (!s->active) return;
     const Rep& R = d.rep[r];
+    const bool active = s->active != 0;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
+    RepState st;
+    Rep Rr;
+    if (active) {
+        if (R.flags & F_PME) {
+            for (int b = threadIdx.x; b < R.pme_blocks; b += blockDim.x) {
+                v[2] += d.pme_part[2 * (R.pme_block_begin + b)];
+                v[3] += d.pme_part[2 * (R.pme_block_begin + b) + 1];
+            }
+        }
+        // one thread uses these: the replica's records copied to registers at
+        // once (independent loads) and written back at the end
+        if (threadIdx.x == 0) {
+            st = *s;
+            Rr = R;
+        }
+    }
+    chain_wait();
+    if (next && r == 0 && threadIdx.x == 0) reset_counters(d);
+    if (!active) return;
     for (int t = R.tile_begin + threadIdx.x; t < R.tile_begin + R.n_tiles; t += blockDim.x) {
         v[0] += d.tile_ke[t];
         v[1] += d.tile_vir[t];
     }
-    if (R.flags & F_PME) {
-        for (int b = threadIdx.x; b < R.pme_blocks; b += blockDim.x) {
-            v[2] += d.pme_part[2 * (R.pme_block_begin + b)];
-            v[3] += d.pme_part[2 * (R.pme_block_begin + b) + 1];
-        }
-    }
     block_sum4(v, sh);
     if (threadIdx.x != 0) return;
-    // one thread from here: the replica's records are copied to registers at
-    // once (independent loads) and written back at the end, instead of a chain
-    // of dependent global reads and writes
-    RepState st = *s;
-    const Rep Rr = R;
     const double ke = v[0], w = v[1];
     st.e_recip = v[2];
     st.vir_recip = v[3];
@@ -693,6 +750,7 @@ __global__ void k_replica_update(Dev d) {
     }
     st.step += 1;
     st.time += dt;
+    if (next) begin_step(st, Rr);
     *s = st;
 }
 
@@ -798,8 +856,8 @@ void launch_rattle(const Dev& d, cudaStream_t st, long long* n) {
     launch_chained(k_tile_ke, (d.n_slots + 255) / 256, 256, st, d);
     *n += 2;
 }
-void launch_replica_update(const Dev& d, cudaStream_t st, long long* n) {
-    launch_chained(k_replica_update, d.n_rep, 256, st, d);
+void launch_replica_update(const Dev& d, bool next, cudaStream_t st, long long* n) {
+    launch_chained(k_replica_update, d.n_rep, 256, st, d, next ? 1 : 0);
     ++*n;
 }
 void launch_apply_scale(const Dev& d, bool, cudaStream_t st, long long* n) {

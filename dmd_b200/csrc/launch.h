@@ -68,7 +68,8 @@ void launch_kick2(const Dev& d, bool andersen_ref, bool andersen_phys, bool chai
                   long long* nlaunch);
 void launch_shake(const Dev& d, cudaStream_t st, long long* nlaunch);
 void launch_rattle(const Dev& d, cudaStream_t st, long long* nlaunch);
-void launch_replica_update(const Dev& d, cudaStream_t st, long long* nlaunch);
+// next: begin the next step too (another step of the same launch follows)
+void launch_replica_update(const Dev& d, bool next, cudaStream_t st, long long* nlaunch);
 void launch_apply_scale(const Dev& d, bool fp64, cudaStream_t st, long long* nlaunch);
 void launch_finalize_velocities(const Dev& d, cudaStream_t st, long long* nlaunch);
 void launch_energy_reduce(const Dev& d, cudaStream_t st, long long* nlaunch);

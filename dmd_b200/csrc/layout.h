@@ -105,6 +105,11 @@ struct RepState {
     int green_ok;         // the cached PME influence function matches the box
     double green_L;       // box edge the cached influence function was made for
     double L_build;       // box edge at the last list build (with xr/yr/zr: the list's frame)
+    // what this step's kick and drift take from the step before (begin_step):
+    double dr_vscale;     // thermostat velocity scale
+    double dr_pscale;     // barostat position scale
+    double dr_L;          // box edge before that scale
+    int dr_move;          // the replica advances
 };
 
 // Kernel view of the whole batch (passed by value).
