@@ -206,6 +206,7 @@ __device__ __forceinline__ void tile_warp(const Dev& d, int t, int lane) {
 // within 1e-5 of the cutoff; PHYS drops excluded pairs.
 constexpr int BW = 4;
 constexpr int NT_B = 32 * BW;
+constexpr int PUSHCAP = 160;    // plain scan: general-path entries buffered per warp before chunks are reserved
 constexpr int MAXC = 48;        // plain scan: candidates per batch
 constexpr int CELL_TILES = 2048;  // replicas with at least this many tiles use cell ranges
 constexpr int MAXR = 128;       // cell ranges: column z-runs per i-tile before the plain scan takes over
@@ -213,7 +214,8 @@ constexpr int OUTCAP = 256;     // cell ranges: entries buffered per warp before
 constexpr int GRP = 4;          // cell ranges: candidate j-tiles whose atoms are loaded together
 constexpr int STAGE = 32 * GRP + 64;  // staged j atoms: < 32 left over + one load group + padding
 constexpr float FAR = 1e18f;  // coordinate of padding atoms: r^2 overflows to +inf
-constexpr int ONE_IMAGE = 1 << 6;
+constexpr int ONE_IMAGE = 1 << 6;  // one periodic image serves every pair of the two tiles
+constexpr int ONE_X = 1 << 7, ONE_Y = 1 << 8, ONE_Z = 1 << 9;  // ... along one axis
 
 // Per-warp scratch of the cell-range builder.
 struct TileScratch {
@@ -243,7 +245,7 @@ __device__ __forceinline__ bool ref_member(const Dev& d, int ai, int aj, double 
 struct ScanScratch {
     float lx[32], ly[32], lz[32];
     int a[32];
-    uint32_t e[BW][64], m[BW][64];  // general path: per-warp entry buffers
+    uint32_t e[BW][PUSHCAP + 32], m[BW][PUSHCAP + 32];  // general path: per-warp entry buffers
     int left[BW];
     int cand[MAXC], cinfo[MAXC];
     float4 coff[MAXC];              // j-tile frame -> i-tile frame (FP32)
@@ -255,6 +257,36 @@ struct ScanScratch {
     int jnext, c0;
 };
 
+// Exclusions are applied to finished masks from the j side: a j atom whose
+// exclusion partners lie in the i-tile clears their bits.  Which j-tiles hold a
+// partner of the i-tile at all is kept as a 64-bit hash over tile numbers, so
+// most groups of j atoms skip the (three dependent) loads.  Testing every pair
+// for a partner's index range and settling the hits one by one was half of
+// the mask time for water and three quarters of it for decane.  (The cell-range
+// builder keeps the range test: its replicas are large, few of its groups have
+// hits, and water 750k's list phase was 3 % slower this way.)
+__device__ __forceinline__ uint64_t excluded_tiles(const Dev& d, int e0, int e1) {
+    uint32_t lo = 0, hi = 0;
+    for (int e = e0; e < e1; ++e) {
+        const int b = (d.slot_of_atom[d.ex_list[e]] >> 5) & 63;
+        if (b < 32) lo |= 1u << b;
+        else hi |= 1u << (b - 32);
+    }
+    return static_cast<uint64_t>(__reduce_or_sync(FULL, lo)) | (static_cast<uint64_t>(__reduce_or_sync(FULL, hi)) << 32);
+}
+
+// Mask m of j atom aj (tile J) over the lanes of i-tile I, less its exclusions.
+__device__ __forceinline__ uint32_t less_exclusions(const Dev& d, uint64_t tiles, uint32_t m, int aj, int J, int I) {
+    if (m && ((tiles >> (J & 63)) & 1u)) {
+        const int e1 = d.ex_start[aj + 1];
+        for (int e = d.ex_start[aj]; e < e1; ++e) {
+            const int sl = d.slot_of_atom[d.ex_list[e]];
+            if ((sl >> 5) == I) m &= ~(1u << (sl & 31));
+        }
+    }
+    return m;
+}
+
 __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch& O) {
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -263,8 +295,8 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
     float(&s_ly)[32] = O.ly;
     float(&s_lz)[32] = O.lz;
     int(&s_a)[32] = O.a;
-    uint32_t(&s_e)[BW][64] = O.e;
-    uint32_t(&s_m)[BW][64] = O.m;
+    uint32_t(&s_e)[BW][PUSHCAP + 32] = O.e;
+    uint32_t(&s_m)[BW][PUSHCAP + 32] = O.m;
     int(&s_left)[BW] = O.left;
     int(&s_cand)[MAXC] = O.cand;
     int(&s_cinfo)[MAXC] = O.cinfo;
@@ -300,39 +332,44 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
     __syncthreads();
     const float hIx = d.thx[I], hIy = d.thy[I], hIz = d.thz[I];
     const int t_end = R.tile_begin + R.n_tiles;
-    // this lane's i atom and (PHYS) its exclusion partners, sorted ascending
+    // this lane's i atom
     const int ai = s_a[lane];
     // a padding i lane sits far away (+FAR), padding j atoms at -FAR: no pair
     const float lix = ai >= 0 ? s_lx[lane] : FAR, liy = ai >= 0 ? s_ly[lane] : FAR,
                 liz = ai >= 0 ? s_lz[lane] : FAR;
-    int iex[8];
-    // exclusion partners span [i_lo, i_lo + i_span]; an empty set never matches
-    int i_e0 = 0, i_e1 = 0, i_lo = 0x7fffffff, i_span = 0;
-    if (phys && ai >= 0) {
-        i_e0 = d.ex_start[ai];
-        i_e1 = d.ex_start[ai + 1];
-        if (i_e1 > i_e0) {
-            i_lo = d.ex_list[i_e0];
-            i_span = d.ex_list[i_e1 - 1] - i_lo;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) iex[k] = (i_e0 + k < i_e1) ? d.ex_list[i_e0 + k] : -1;
+    uint64_t ex_tiles = 0;
+    if (phys) ex_tiles = excluded_tiles(d, ai >= 0 ? d.ex_start[ai] : 0, ai >= 0 ? d.ex_start[ai + 1] : 0);
 
     // ---- general path (several periodic images per tile pair) ----------------
     int nbuf = 0;  // entries buffered in s_e/s_m[wib] (warp-uniform)
-    auto flush_chunk = [&](const uint32_t* be, const uint32_t* bm, int count) {
-        int c = 0;
-        if (lane == 0) c = atomicAdd(&s->n_chunks, 1);
-        c = __shfl_sync(FULL, c, 0);
-        if (c >= R.chunk_cap) {
-            if (lane == 0) set_status(s, ST_CAPACITY);
-            return;
+    // the first `count` buffered entries as chunks, the last one padded
+    auto flush_chunks = [&](int count) {
+        const int k = (count + 31) >> 5;
+        int c0 = 0;
+        if (lane == 0) c0 = atomicAdd(&s->n_chunks, k);
+        c0 = __shfl_sync(FULL, c0, 0);
+        if (c0 + k > R.chunk_cap && lane == 0) set_status(s, ST_CAPACITY);
+        for (int q = 0; q < k && c0 + q < R.chunk_cap; ++q) {
+            const int g = R.chunk_begin + c0 + q, idx = 32 * q + lane;
+            if (lane == 0) d.chunk_itile[g] = I;
+            d.chunk_j[32 * g + lane] = idx < count ? s_e[wib][idx] : 0u;
+            d.chunk_mask[32 * g + lane] = idx < count ? s_m[wib][idx] : 0u;
         }
-        const int g = R.chunk_begin + c;
-        if (lane == 0) d.chunk_itile[g] = I;
-        d.chunk_j[32 * g + lane] = lane < count ? be[lane] : 0u;
-        d.chunk_mask[32 * g + lane] = lane < count ? bm[lane] : 0u;
+        __syncwarp();
+        // fewer than 32 entries are left after whole chunks
+        const int left = max(nbuf - count, 0);
+        uint32_t te = 0u, tm = 0u;
+        if (lane < left) {
+            te = s_e[wib][count + lane];
+            tm = s_m[wib][count + lane];
+        }
+        __syncwarp();
+        if (lane < left) {
+            s_e[wib][lane] = te;
+            s_m[wib][lane] = tm;
+        }
+        nbuf = left;
+        __syncwarp();
     };
     auto push = [&](uint32_t e, uint32_t m) {
         const uint32_t has = __ballot_sync(FULL, m != 0);
@@ -343,89 +380,112 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
         }
         nbuf += __popc(has);
         __syncwarp();
-        if (nbuf >= 32) {
-            flush_chunk(s_e[wib], s_m[wib], 32);
-            __syncwarp();
-            if (lane < nbuf - 32) {
-                s_e[wib][lane] = s_e[wib][lane + 32];
-                s_m[wib][lane] = s_m[wib][lane + 32];
+        if (nbuf >= PUSHCAP) flush_chunks(PUSHCAP);
+    };
+    // One candidate tile J whose pairs need several periodic images, lane = j
+    // atom: each j is tested against every i, and every image code found
+    // becomes its own entry (codes in the order of their first i).  The 32
+    // tests are branch-free and leave bit masks over i (inside, and per axis
+    // which way the pair wrapped); cutoff-band pairs and exclusions, both rare,
+    // are settled on the masks.  In boxes of a few cutoffs most tile pairs come
+    // here and the tile with the most of them is the rebuild's critical path:
+    // with a loop over i that branched on every test, a search of the exclusions
+    // per pair and a counter update per chunk, the list phase took 210 us for
+    // water 9k, 155 us for 522 rigid waters, 80 us for argon 4k and 93 us for
+    // decane 4k; now 86, 42, 27 and 42 us.
+    const uint32_t i_valid = __ballot_sync(FULL, ai >= 0);
+    // one axis of eight tests: r2[q] += (wrapped) displacement^2; an axis whose
+    // extents stay inside half a box (`one`, the same for the warp) cannot wrap
+    auto general_axis = [&](const float* li, float jc, bool one, int i0, float (&r2)[8], uint32_t& p, uint32_t& m) {
+        if (one) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float dc = jc - li[i0 + q];
+                r2[q] = fmaf(dc, dc, r2[q]);
             }
-            nbuf -= 32;
-            __syncwarp();
+        } else {
+            uint32_t p8 = 0, m8 = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                float dc = jc - li[i0 + q];
+                const bool up = dc > hLf, dn = dc < -hLf;
+                dc += up ? -Lf : (dn ? Lf : 0.f);
+                p8 |= static_cast<uint32_t>(up) << q;
+                m8 |= static_cast<uint32_t>(dn) << q;
+                r2[q] = fmaf(dc, dc, r2[q]);
+            }
+            p |= p8 << i0;
+            m |= m8 << i0;
         }
     };
-    // One candidate tile J, lane = j atom: each j is tested against every i,
-    // and every periodic image code found becomes its own entry.
-    auto general_candidate = [&](int J) {
-        const int js = 32 * J + lane;
-        const int aj = d.atom_of_slot[js];
-        const double ddx = d.tcx[J] - cIx, ddy = d.tcy[J] - cIy, ddz = d.tcz[J] - cIz;
-        const double rx0 = round(ddx * invL), ry0 = round(ddy * invL), rz0 = round(ddz * invL);
-        float jx = 0.f, jy = 0.f, jz = 0.f;
-        int ex[8];
-        int nex = 0, e0 = 0, e1 = 0;
-        if (aj >= 0) {
-            jx = static_cast<float>((d.x[aj] - d.imgx[aj] * L) - cIx - rx0 * L);
-            jy = static_cast<float>((d.y[aj] - d.imgy[aj] * L) - cIy - ry0 * L);
-            jz = static_cast<float>((d.z[aj] - d.imgz[aj] * L) - cIz - rz0 * L);
-            e0 = d.ex_start[aj];
-            e1 = d.ex_start[aj + 1];
-            if (phys) nex = e1 - e0;
-        }
+    // k: index of the candidate; pj, aj: this lane's j atom (build frame of its tile)
+    auto general_candidate = [&](int k, float4 pj, int aj) {
+        const int J = s_cand[k], info = s_cinfo[k], js = 32 * J + lane;
+        const int rx0 = (info & 3) - 1, ry0 = ((info >> 2) & 3) - 1, rz0 = ((info >> 4) & 3) - 1;
+        const float4 o = s_coff[k];
+        const float jx = pj.x + o.x, jy = pj.y + o.y, jz = pj.z + o.z;
+        const uint32_t todo = aj >= 0 ? i_valid & ((J == I) ? ((1u << lane) - 1u) : 0xffffffffu) : 0u;
+        uint32_t in = 0, band = 0, xp = 0, xm = 0, yp = 0, ym = 0, zp = 0, zm = 0;
+#pragma unroll 1
+        for (int i0 = 0; i0 < 32; i0 += 8) {
+            float r2[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            general_axis(s_lx, jx, info & ONE_X, i0, r2, xp, xm);
+            general_axis(s_ly, jy, info & ONE_Y, i0, r2, yp, ym);
+            general_axis(s_lz, jz, info & ONE_Z, i0, r2, zp, zm);
+            uint32_t in8 = 0, b8 = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) ex[k] = (k < nex) ? d.ex_list[e0 + k] : -1;
-        uint32_t todo = 0;
-        if (aj >= 0) todo = (J == I) ? ((1u << lane) - 1u) : 0xffffffffu;
-        while (__any_sync(FULL, todo != 0)) {
-            uint32_t bits = 0, rest = 0, code0 = 0xffffffffu;
-            for (uint32_t t = todo; t; t &= t - 1) {
-                const int i = __ffs(t) - 1;
-                const int a_i = s_a[i];
-                if (a_i < 0) continue;
-                float dx = jx - s_lx[i], dy = jy - s_ly[i], dz = jz - s_lz[i];
-                int sx = 0, sy = 0, sz = 0;
-                if (dx > hLf) { dx -= Lf; sx = 1; } else if (dx < -hLf) { dx += Lf; sx = -1; }
-                if (dy > hLf) { dy -= Lf; sy = 1; } else if (dy < -hLf) { dy += Lf; sy = -1; }
-                if (dz > hLf) { dz -= Lf; sz = 1; } else if (dz < -hLf) { dz += Lf; sz = -1; }
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 >= rc2_hi) continue;
-                int mx, my, mz;
-                if (r2 > rc2_lo) {
-                    // borderline: the reference's FP64 expression decides
-                    double ex_ = __dsub_rn(d.x[aj], d.x[a_i]), ey = __dsub_rn(d.y[aj], d.y[a_i]),
-                           ez = __dsub_rn(d.z[aj], d.z[a_i]);
-                    const double qx = round(__dmul_rn(ex_, invL)), qy = round(__dmul_rn(ey, invL)),
-                                 qz = round(__dmul_rn(ez, invL));
-                    ex_ = __dsub_rn(ex_, __dmul_rn(qx, L));
-                    ey = __dsub_rn(ey, __dmul_rn(qy, L));
-                    ez = __dsub_rn(ez, __dmul_rn(qz, L));
-                    if (!(r2_ref(ex_, ey, ez) < rc2)) continue;
-                    mx = d.imgx[aj] - d.imgx[a_i] - static_cast<int>(qx);
-                    my = d.imgy[aj] - d.imgy[a_i] - static_cast<int>(qy);
-                    mz = d.imgz[aj] - d.imgz[a_i] - static_cast<int>(qz);
-                } else {
-                    // displacement = w_j - w_i - (r0 + s) L
-                    mx = -static_cast<int>(rx0) - sx;
-                    my = -static_cast<int>(ry0) - sy;
-                    mz = -static_cast<int>(rz0) - sz;
-                }
-                if (phys) {
-                    bool excluded = false;
-                    if (nex <= 8) {
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) excluded |= (ex[k] == a_i);
-                    } else {
-                        for (int e = e0; e < e1; ++e) excluded |= (d.ex_list[e] == a_i);
-                    }
-                    if (excluded) continue;
-                }
-                const uint32_t code = static_cast<uint32_t>((mx + 1) | ((my + 1) << 2) | ((mz + 1) << 4));
-                if (code0 == 0xffffffffu) code0 = code;
-                if (code == code0) bits |= 1u << i;
-                else rest |= 1u << i;
+            for (int q = 0; q < 8; ++q) {
+                const bool near = !(r2[q] >= rc2_hi);
+                in8 |= static_cast<uint32_t>(near) << q;
+                b8 |= static_cast<uint32_t>(near & (r2[q] > rc2_lo)) << q;
             }
-            push(static_cast<uint32_t>(js) | ((bits ? code0 : 0u) << 26), bits);
-            todo = rest;
+            in |= in8 << i0;
+            band |= b8 << i0;
+        }
+        in &= todo;
+        in = less_exclusions(d, ex_tiles, in, aj, J, I);
+        band &= in;
+        while (band) {  // borderline: the reference's FP64 expression decides
+            const int i = __ffs(band) - 1;
+            const uint32_t b = 1u << i;
+            band &= band - 1;
+            const int a_i = s_a[i];
+            double ex_ = __dsub_rn(d.x[aj], d.x[a_i]), ey = __dsub_rn(d.y[aj], d.y[a_i]),
+                   ez = __dsub_rn(d.z[aj], d.z[a_i]);
+            const double qx = round(__dmul_rn(ex_, invL)), qy = round(__dmul_rn(ey, invL)),
+                         qz = round(__dmul_rn(ez, invL));
+            ex_ = __dsub_rn(ex_, __dmul_rn(qx, L));
+            ey = __dsub_rn(ey, __dmul_rn(qy, L));
+            ez = __dsub_rn(ez, __dmul_rn(qz, L));
+            if (!(r2_ref(ex_, ey, ez) < rc2)) {
+                in &= ~b;
+                continue;
+            }
+            // displacement = w_j - w_i - (r0 + s) L
+            const int sx = static_cast<int>(qx) - d.imgx[aj] + d.imgx[a_i] - rx0;
+            const int sy = static_cast<int>(qy) - d.imgy[aj] + d.imgy[a_i] - ry0;
+            const int sz = static_cast<int>(qz) - d.imgz[aj] + d.imgz[a_i] - rz0;
+            xp = sx > 0 ? xp | b : xp & ~b;
+            xm = sx < 0 ? xm | b : xm & ~b;
+            yp = sy > 0 ? yp | b : yp & ~b;
+            ym = sy < 0 ? ym | b : ym & ~b;
+            zp = sz > 0 ? zp | b : zp & ~b;
+            zm = sz < 0 ? zm | b : zm & ~b;
+        }
+        while (__any_sync(FULL, in != 0)) {
+            uint32_t bits = 0, code = 0;
+            if (in) {
+                const int i = __ffs(in) - 1;
+                const int sx = static_cast<int>((xp >> i) & 1u) - static_cast<int>((xm >> i) & 1u);
+                const int sy = static_cast<int>((yp >> i) & 1u) - static_cast<int>((ym >> i) & 1u);
+                const int sz = static_cast<int>((zp >> i) & 1u) - static_cast<int>((zm >> i) & 1u);
+                bits = in & (sx > 0 ? xp : ~xp) & (sx < 0 ? xm : ~xm) & (sy > 0 ? yp : ~yp) &
+                       (sy < 0 ? ym : ~ym) & (sz > 0 ? zp : ~zp) & (sz < 0 ? zm : ~zm);
+                const int mx = -rx0 - sx, my = -ry0 - sy, mz = -rz0 - sz;
+                code = static_cast<uint32_t>((mx + 1) | ((my + 1) << 2) | ((mz + 1) << 4));
+                in &= ~bits;
+            }
+            push(static_cast<uint32_t>(js) | (code << 26), bits);
         }
     };
 
@@ -460,9 +520,10 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
                 // one periodic image serves every pair of the two tiles when their
                 // extents around the centre displacement stay inside half a box
                 const double hL = 0.5 * L;
-                const bool one = fabs(dx) + ex < hL && fabs(dy) + ey < hL && fabs(dz) + ez < hL;
+                const bool one_x = fabs(dx) + ex < hL, one_y = fabs(dy) + ey < hL, one_z = fabs(dz) + ez < hL;
                 info[u] = (static_cast<int>(rx0) + 1) | ((static_cast<int>(ry0) + 1) << 2) |
-                          ((static_cast<int>(rz0) + 1) << 4) | (one ? ONE_IMAGE : 0);
+                          ((static_cast<int>(rz0) + 1) << 4) | ((one_x && one_y && one_z) ? ONE_IMAGE : 0) |
+                          (one_x ? ONE_X : 0) | (one_y ? ONE_Y : 0) | (one_z ? ONE_Z : 0);
                 off[u] = make_float4(static_cast<float>(dx), static_cast<float>(dy), static_cast<float>(dz), 0.f);
             }
             uint32_t bal[4];
@@ -515,13 +576,12 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
                 if (!(info & ONE_IMAGE)) continue;
                 const int js = 32 * s_cand[k] + (idx & 31);
                 const int aj = d.atom_of_slot[js];
-                if (aj < 0) continue;
-                const float4 p = d.xl32[js];
+                const float4 p = d.xl32[js];  // (both loads in flight together)
                 const float4 o = s_coff[k];
                 pj[u] = make_float4(p.x + o.x, p.y + o.y, p.z + o.z, __int_as_float(aj));
                 const float gx = fmaxf(fabsf(pj[u].x) - hIx, 0.f), gy = fmaxf(fabsf(pj[u].y) - hIy, 0.f),
                             gz = fmaxf(fabsf(pj[u].z) - hIz, 0.f);
-                keep[u] = gx * gx + gy * gy + gz * gz <= rc2_hi * 1.0001f + 1e-6f;
+                keep[u] = aj >= 0 && gx * gx + gy * gy + gz * gz <= rc2_hi * 1.0001f + 1e-6f;
                 const uint32_t code = static_cast<uint32_t>((2 - (info & 3)) | ((2 - ((info >> 2) & 3)) << 2) |
                                                             ((2 - ((info >> 4) & 3)) << 4));
                 ent[u] = static_cast<uint32_t>(js) | (code << 26);
@@ -559,46 +619,60 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
         }
         __syncthreads();
         // 3. masks, 32 staged j atoms per warp pass; lane = i atom, one ballot per
-        //    j.  Pairs at the cutoff band or among the i atom's exclusion partners
-        //    are settled after the pass (rare): FP64 reference test, exclusions.
+        //    j.  Pairs in the cutoff band (rare) are settled after the pass by the
+        //    FP64 reference test, then the exclusions are taken out.
         for (int g = wib; g < ngroups; g += BW) {
             const float4* pjs = s_jx + 32 * g;
             uint32_t rare = 0;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 const float4 pj = pjs[j];
-                const int a2 = __float_as_int(pj.w);
                 const float dx = pj.x - lix, dy = pj.y - liy, dz = pj.z - liz;
                 const float r2 = dx * dx + dy * dy + dz * dz;
-                const bool exr = static_cast<unsigned>(a2 - i_lo) <= static_cast<unsigned>(i_span);
-                const bool in = (r2 < rc2_lo) & !exr;
-                rare |= static_cast<uint32_t>((r2 < rc2_hi) & ((r2 >= rc2_lo) | exr)) << j;
-                const uint32_t m = __ballot_sync(FULL, in);
+                rare |= static_cast<uint32_t>((r2 < rc2_hi) & (r2 >= rc2_lo)) << j;
+                const uint32_t m = __ballot_sync(FULL, r2 < rc2_lo);
                 if (lane == 0) s_msk[32 * g + j] = m;
             }
             __syncwarp();
             while (rare) {
                 const int j = __ffs(rare) - 1;
                 rare &= rare - 1;
-                const float4 pj = pjs[j];
-                const int a2 = __float_as_int(pj.w);
-                const float dx = pj.x - lix, dy = pj.y - liy, dz = pj.z - liz;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                bool in = (r2 < rc2_lo) || ref_member(d, ai, a2, L, invL, rc2);
-                if (in && static_cast<unsigned>(a2 - i_lo) <= static_cast<unsigned>(i_span)) {
-                    if (i_e1 - i_e0 <= 8) {
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) in &= (iex[q] != a2);
-                    } else {
-                        for (int e = i_e0; e < i_e1; ++e) in &= (d.ex_list[e] != a2);
-                    }
-                }
-                if (in) atomicOr(&s_msk[32 * g + j], 1u << lane);
+                if (ref_member(d, ai, __float_as_int(pjs[j].w), L, invL, rc2)) atomicOr(&s_msk[32 * g + j], 1u << lane);
+            }
+            __syncwarp();
+            if (ex_tiles) {
+                const int js = static_cast<int>(s_je[32 * g + lane] & 0x03FFFFFFu);
+                const uint32_t m = s_msk[32 * g + lane];
+                s_msk[32 * g + lane] = less_exclusions(d, ex_tiles, m, __float_as_int(pjs[lane].w), js >> 5, I);
             }
         }
         // general path for candidates that need several periodic images
-        for (int k = wib; k < nc; k += BW)
-            if (!(s_cinfo[k] & ONE_IMAGE)) general_candidate(s_cand[k]);
+        // (the next one's j atoms are in flight while one is tested)
+        {
+            auto next_general = [&](int k) {
+                while (k < nc && (s_cinfo[k] & ONE_IMAGE)) k += BW;
+                return k;
+            };
+            int k = next_general(wib), aj = -1;
+            float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < nc) {
+                aj = d.atom_of_slot[32 * s_cand[k] + lane];
+                pj = d.xl32[32 * s_cand[k] + lane];
+            }
+            while (k < nc) {
+                const int k2 = next_general(k + BW);
+                int aj2 = -1;
+                float4 pj2 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k2 < nc) {
+                    aj2 = d.atom_of_slot[32 * s_cand[k2] + lane];
+                    pj2 = d.xl32[32 * s_cand[k2] + lane];
+                }
+                general_candidate(k, pj, aj);
+                k = k2;
+                aj = aj2;
+                pj = pj2;
+            }
+        }
         __syncthreads();
         // 4. ordered compaction of the non-empty entries (s_jx reused), whole chunks out
         uint32_t* s_oe = reinterpret_cast<uint32_t*>(s_jx);
@@ -661,18 +735,17 @@ __device__ __forceinline__ void build_tile_scan(const Dev& d, int I, ScanScratch
         __syncthreads();
     }
     // merge the carry and the general path's leftovers: warp 0 flushes them
+    if (nbuf >= 32) flush_chunks(nbuf & ~31);
     if (lane == 0) s_left[wib] = nbuf;
     __syncthreads();
     if (wib == 0) {
         for (int w = 1; w < BW; ++w) {
             const int nl = s_left[w];
-            for (int base = 0; base < nl; base += 32) {
-                const bool mine = base + lane < nl;
-                push(mine ? s_e[w][base + lane] : 0u, mine ? s_m[w][base + lane] : 0u);
-            }
+            const bool mine = lane < nl;
+            push(mine ? s_e[w][lane] : 0u, mine ? s_m[w][lane] : 0u);
         }
         push(lane < carry_n ? s_carry_e[lane] : 0u, lane < carry_n ? s_carry_m[lane] : 0u);
-        if (nbuf > 0) flush_chunk(s_e[0], s_m[0], nbuf);
+        if (nbuf > 0) flush_chunks(nbuf);
     }
 }
 

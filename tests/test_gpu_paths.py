@@ -53,3 +53,32 @@ def test_constraint_paths(oracle, n_mol, order):
     eng.run_n(6)
     assert np.abs(eng.positions - oe.get(0)).max() / c.box_size < 1e-8
     assert rel_rms(eng.velocities, oe.get(1)) < 1e-8
+
+
+def _lists(cfg, oracle, profile):
+    eng = _engine(cfg, "mixed", profile)
+    eng.compute_forces()
+    got = eng.pair_list()
+    return set(zip(*[a.tolist() for a in got])), eng
+
+
+@pytest.mark.parametrize("profile", ["ref", "phys"])
+@pytest.mark.parametrize("n_chains", [9, 26, 40, 130])
+def test_pair_set_several_images_and_exclusions(oracle, n_chains, profile):
+    """List build in boxes of one to three cutoffs (tile pairs that need several
+    periodic images, along one, two or three axes) with chain exclusions that
+    reach into neighbouring tiles: the pair set equals a brute-force FP64 one."""
+    cfg = W.decane_melt(n_chains, 3).config()
+    got, eng = _lists(cfg, oracle, profile)
+    x = np.stack([cfg.pos_x, cfg.pos_y, cfg.pos_z], 1)
+    L = cfg.box_size
+    rc = cfg.lj_cutoff + (0.15 if profile == "phys" else 0.0)
+    ex = {(min(i, j), max(i, j)) for i, j in zip(cfg.excl_i, cfg.excl_j)} if profile == "phys" else set()
+    want = set()
+    for i in range(len(x) - 1):
+        dd = x[i + 1:] - x[i]
+        q = dd * (1.0 / L)
+        dd = dd - np.copysign(np.floor(np.abs(q) + 0.5), q) * L
+        r2 = dd[:, 0] * dd[:, 0] + dd[:, 1] * dd[:, 1] + dd[:, 2] * dd[:, 2]
+        want.update((i, int(j)) for j in np.nonzero(r2 < rc * rc)[0] + i + 1)
+    assert got == want - ex
