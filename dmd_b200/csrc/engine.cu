@@ -125,6 +125,59 @@ void sort_grid(int n, double L, int& nvx, int& nvz) {
 
 }  // namespace
 
+// Coefficients (powers of u = 2 r^2 / rc^2 - 1) of
+//   P(r^2) = erf(a r) / r^3 - 2 a / sqrt(pi) exp(-a^2 r^2) / r^2
+//          = a^3 (4 / sqrt(pi)) int_0^1 t^2 exp(-a^2 r^2 t^2) dt,
+// by Chebyshev interpolation in extended precision; false when EWALD_N of them
+// do not reach FP64 rounding (a rc above about 3.3) or the cutoff is not usable.
+static bool ewald_polynomial(double alpha, double rc, double* out) {
+    using ld = long double;
+    constexpr int N = EWALD_N;
+    const ld pi = 3.141592653589793238462643383279502884L;
+    const ld a = alpha, S = a * a * static_cast<ld>(rc) * rc;
+    if (!(alpha > 0.0) || !(rc > 0.0) || !(S < 64.0L)) return false;
+    auto f = [&](ld s) -> ld {  // s = a^2 r^2
+        if (s < 2.0L) {
+            ld sum = 0.0L, term = 1.0L;  // sum over (-s)^n / (n! (2n + 3))
+            for (int n = 0; n < 60; ++n) {
+                sum += term / (2 * n + 3);
+                term *= -s / (n + 1);
+            }
+            return a * a * a * 4.0L / sqrtl(pi) * sum;
+        }
+        const ld x = sqrtl(s);
+        return a * a * a * (erfl(x) / (s * x) - 2.0L / sqrtl(pi) * expl(-s) / s);
+    };
+    ld c[N], v[N];
+    for (int k = 0; k < N; ++k) v[k] = f(0.5L * S * (1.0L + cosl(pi * (k + 0.5L) / N)));
+    for (int n = 0; n < N; ++n) {
+        ld sum = 0.0L;
+        for (int k = 0; k < N; ++k) sum += v[k] * cosl(pi * n * (k + 0.5L) / N);
+        c[n] = sum * (n ? 2.0L : 1.0L) / N;
+    }
+    ld mono[N] = {}, t0[N] = {}, t1[N] = {};
+    t0[0] = 1.0L;
+    t1[1] = 1.0L;
+    for (int n = 0; n < N; ++n) {
+        for (int k = 0; k < N; ++k) mono[k] += c[n] * t0[k];
+        ld t2[N];
+        for (int k = 0; k < N; ++k) t2[k] = (k ? 2.0L * t1[k - 1] : 0.0L) - t0[k];
+        for (int k = 0; k < N; ++k) {
+            t0[k] = t1[k];
+            t1[k] = t2[k];
+        }
+    }
+    for (int k = 0; k < N; ++k) out[k] = static_cast<double>(mono[k]);
+    ld worst = 0.0L;
+    for (int k = 0; k <= 400; ++k) {
+        const ld u = -1.0L + k / 200.0L;
+        double q = out[N - 1];
+        for (int n = N - 2; n >= 0; --n) q = std::fma(q, static_cast<double>(u), out[n]);
+        worst = std::max(worst, fabsl(static_cast<ld>(q) - f(0.5L * S * (1.0L + u))));
+    }
+    return worst < 1e-15L * f(0.0L);
+}
+
 // ---------------------------------------------------------------------------
 // Autotuner cache: the pair kernel's launch shape chosen for a kind of batch,
 // shared by every batch of the process (the serving loop repacks often).
@@ -838,6 +891,7 @@ int Batch::pack() {
         std::vector<int> pbr(std::max(pme_blocks, 1));
         std::vector<int> cbr(std::max(conv_blocks, 1));
         std::vector<Rep> hrep(R);
+        std::vector<double> hew(fp64_ ? static_cast<size_t>(R) * EWALD_N : 0);
         for (int k = 0; k < R; ++k) {
             HostRep& h = *reps_[order_[k]];
             HostSystem& s = h.sys;
@@ -966,6 +1020,7 @@ int Batch::pack() {
                 for (int b = 0; b < P.pme_blocks; ++b) pbr[P.pme_block_begin + b] = k;
                 for (int b = 0; b < P.conv_blocks; ++b) cbr[P.conv_block_begin + b] = k;
             }
+            P.ewald_ok = fp64_ && (P.flags & F_COUL_REAL) && ewald_polynomial(P.alpha, P.rc_c, &hew[EWALD_N * k]) ? 1 : 0;
             hrep[k] = P;
         }
         // exclusion CSR: each atom's excluded partners, ascending, without
@@ -1012,6 +1067,11 @@ int Batch::pack() {
         up(d.xr, hxr.data(), 8 * n_atoms);
         up(d.yr, hyr.data(), 8 * n_atoms);
         up(d.zr, hzr.data(), 8 * n_atoms);
+        if (fp64_) {
+            double* ew = A.alloc<double>(hew.size());
+            up(ew, hew.data(), 8 * hew.size());
+            d.ewald_poly = ew;
+        }
         up(mass, hm.data(), 8 * n_atoms);
         up(q, hq.data(), 8 * n_atoms);
         up(type, ht.data(), 4 * n_atoms);
@@ -1400,6 +1460,7 @@ constexpr int kManyAtoms = 400000;
 int Batch::run_steps(int n) {
     st_fresh_ = false;  // device work follows: the host mirror is stale
     if (n <= 0) return DMDGPU_OK;
+    if (fp64_) launch_mark_read(dev_, n, stream_, &launches_);
     static const bool eager = [] {
         const char* e = std::getenv("DMD_EAGER");
         return e && e[0] == '1';
@@ -1832,6 +1893,7 @@ int Batch::step_timed(int n, long long flush_bytes, dmdgpu_timing* out) {
         CK(cudaMalloc(&flush_buf_, flush_bytes));
         flush_bytes_ = flush_bytes;
     }
+    if (fp64_) launch_mark_read(dev_, n, stream_, &launches_);
     // capture one step with its pair-kernel and PME events
     ev_used_ = 0;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> nb0, pme0;

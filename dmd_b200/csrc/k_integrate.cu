@@ -70,9 +70,10 @@ __device__ __forceinline__ void begin_step(RepState& s, const Rep& R) {
         s.pscale = 1.0;
     }
     // Pair energies and the pair virial are needed by single-point evaluations,
-    // by the evaluation that ends a run (its energies are what the host reads) and,
-    // with the PHYS barostat, every step (its pressure uses the atomic virial).
-    begin_eval(s, R, s.active, s.step + 1 >= s.target_step || ((R.flags & F_PHYS) && R.barostat));
+    // by the evaluation that ends a run (its energies are what the host reads; the
+    // FP64 path forms them at the end of every call, read_step) and, with the PHYS
+    // barostat, every step (its pressure uses the atomic virial).
+    begin_eval(s, R, s.active, s.step + 1 >= s.target_step || s.step + 1 == s.read_step || ((R.flags & F_PHYS) && R.barostat));
 }
 
 __global__ void k_eval_begin(Dev d, int pass) {
@@ -102,6 +103,12 @@ __global__ void k_eval_begin(Dev d, int pass) {
     }
     // eval #1 never needs energies: eval #2 of the same step overwrites its sums
     begin_eval(*s, R, ev, pass == PASS_SINGLE);
+}
+
+// FP64: the replicas' energies are read after n more steps.
+__global__ void k_mark_read(Dev d, int n) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < d.n_rep) d.st[r].read_step = d.st[r].step + n;
 }
 
 __global__ void k_eval_end(Dev d) {
@@ -826,6 +833,10 @@ __global__ void k_write_mirror(Dev d) {
 
 void launch_eval_begin(const Dev& d, int pass, cudaStream_t st, long long* n) {
     launch_chained(k_eval_begin, (d.n_rep + 127) / 128, 128, st, d, pass);
+    ++*n;
+}
+void launch_mark_read(const Dev& d, int n_steps, cudaStream_t st, long long* n) {
+    k_mark_read<<<(d.n_rep + 127) / 128, 128, 0, st>>>(d, n_steps);
     ++*n;
 }
 void launch_clear_forces(const Dev& d, cudaStream_t st, long long* n) {

@@ -682,105 +682,304 @@ __global__ void __launch_bounds__(256, 2) k_nb8_f32(Dev d) {
     flush_acc(d, cur, acc);
 }
 
+// ---- all-FP64 path ----------------------------------------------------------
+// Per-warp staging of one chunk's j entries.
+struct ChunkStage64 {
+    double4 xq[32];
+    int tj[32];
+    int js[32];
+    uint32_t mk[32];
+};
+
+// One chunk of a replica whose Ewald polynomial does not apply (alpha rc beyond
+// what EWALD_N coefficients reach): erfc() and exp() for the real-space Ewald
+// term, LJ in the reference's operation order, the minimum image taken per pair
+// with the reference's expression.
+__device__ __noinline__ void nb_chunk_f64_erfc(const Dev& d, const Rep& R, RepState* s, int c, int lane, ChunkStage64& S,
+                                          Acc& acc) {
+    const double L = s->L, invL = s->invL;
+    const int I = d.chunk_itile[c];
+    const int si = 32 * I + lane;
+    const double4 xi = d.xq64[si];
+    const int ti = d.type_s[si];
+    const uint32_t e = d.chunk_j[32 * c + lane];
+    const uint32_t mk = d.chunk_mask[32 * c + lane];
+    const int js = static_cast<int>(e & 0x03FFFFFFu);
+    double4 xj = make_double4(0, 0, 0, 0);
+    int tj = 0;
+    if (mk) {
+        xj = d.xq64[js];
+        tj = d.type_s[js];
+    }
+    S.xq[lane] = xj;
+    S.tj[lane] = tj;
+    S.mk[lane] = mk;
+    __syncwarp();
+    const bool has_lj = (R.flags & F_LJ) != 0;
+    const bool has_c = (R.flags & F_COUL_REAL) != 0;
+    const double rl2 = R.rc_lj2, rcc2 = R.rc_c2, alpha = R.alpha;
+    const double2* lj = d.lj64 + R.lj_off + ti * R.n_types;
+    double fix = 0, fiy = 0, fiz = 0, fjx = 0, fjy = 0, fjz = 0;
+    double el = 0, ec = 0, vir = 0;
+    for (int k = 0; k < 32; ++k) {
+        const int src = (lane + k) & 31;
+        const uint32_t m = S.mk[src];
+        if ((m >> lane) & 1u) {
+            const double4 pj = S.xq[src];
+            const double dx = mi_ref(__dsub_rn(pj.x, xi.x), L, invL);
+            const double dy = mi_ref(__dsub_rn(pj.y, xi.y), L, invL);
+            const double dz = mi_ref(__dsub_rn(pj.z, xi.z), L, invL);
+            const double r2 = r2_ref(dx, dy, dz);
+            double f = 0.0;
+            if (has_lj && r2 < rl2) {
+                // 24 eps (2 sr6^2 - sr6) / r2 and 4 eps (sr6^2 - sr6), reference order
+                const double2 p = lj[S.tj[src]];
+                const double r6 = __dmul_rn(__dmul_rn(r2, r2), r2);
+                const double sr6 = __ddiv_rn(p.y, r6);
+                f = __ddiv_rn(__dmul_rn(__dmul_rn(24.0, p.x),
+                                        __dsub_rn(__dmul_rn(__dmul_rn(2.0, sr6), sr6), sr6)), r2);
+                el += __dmul_rn(__dmul_rn(4.0, p.x), __dsub_rn(__dmul_rn(sr6, sr6), sr6));
+            }
+            if (has_c && r2 < rcc2) {
+                const double qq = KE * xi.w * pj.w;
+                const double r = sqrt(r2);
+                const double erfc_ar = erfc(alpha * r);
+                f += qq * (erfc_ar / (r2 * r) + 2.0 * alpha * exp(-alpha * alpha * r2) /
+                                                    (1.7724538509055160273 * r2));
+                ec += qq * erfc_ar / r;
+            }
+            vir += f * r2;
+            fix -= f * dx;
+            fiy -= f * dy;
+            fiz -= f * dz;
+            fjx += f * dx;
+            fjy += f * dy;
+            fjz += f * dz;
+        }
+        fjx = __shfl_sync(FULL, fjx, (lane + 1) & 31);
+        fjy = __shfl_sync(FULL, fjy, (lane + 1) & 31);
+        fjz = __shfl_sync(FULL, fjz, (lane + 1) & 31);
+    }
+    if (d.atom_of_slot[si] >= 0) {
+        fix_add(d.fnx + si, to_fix(fix, FSCALE, s));
+        fix_add(d.fny + si, to_fix(fiy, FSCALE, s));
+        fix_add(d.fnz + si, to_fix(fiz, FSCALE, s));
+    }
+    if (mk) {
+        fix_add(d.fnx + js, to_fix(fjx, FSCALE, s));
+        fix_add(d.fny + js, to_fix(fjy, FSCALE, s));
+        fix_add(d.fnz + js, to_fix(fjz, FSCALE, s));
+    }
+    acc.lj += to_fix(el, ESCALE, s);
+    acc.c += to_fix(ec, ESCALE, s);
+    acc.v += to_fix(vir, ESCALE, s);
+    __syncwarp();
+}
+
+// 1 / sqrt(x), x > 0: the single-precision approximation and one Halley step
+// (cubic: its ~2^-22 relative error becomes ~2^-65, below rounding).
+__device__ __forceinline__ double rsqrt_h(double x) {
+    const double y = static_cast<double>(rsqrt_ap(static_cast<float>(x)));
+    const double h = fma(-x * y, y, 1.0);
+    return fma(y * h, fma(h, 0.375, 0.5), y);
+}
+
+// One chunk.  Bound by the FP64 pipe, so by what a pair costs in
+// it: a list entry's periodic image is the one frozen at the build (MI: the
+// box is narrower than twice the list cutoff, nearest image per pair), LJ and
+// the Ewald term share one reciprocal square root, and the Ewald term
+//   erfc(a r) / r^3 + 2 a / sqrt(pi) exp(-a^2 r^2) / r^2 = r^-3 - P(r^2)
+// with P(r^2) = erf(a r) / r^3 - 2 a / sqrt(pi) exp(-a^2 r^2) / r^2, which is
+// smooth in r^2 down to 0, as a polynomial fitted for the replica (EWALD_N
+// coefficients in registers) -- instead of a root, five divisions, erfc() and
+// exp().  Membership is the reference's: a pair within 1e-12 (relative) of a
+// cutoff is decided by its expression.  Energies (ENERGY) are formed beside the
+// same force arithmetic, with erfc(), so a force does not depend on whether its
+// evaluation's energies are read.  Water 30k, 22,800 chunks: 560 -> 177
+// us per launch.
+template <bool COUL, bool MI, bool ENERGY>
+__device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
+                                             ChunkStage64& S, Acc& acc) {
+    const double L = s->L, invL = s->invL;
+    const int I = d.chunk_itile[c];
+    const int si = 32 * I + lane;
+    double4 xi = d.xq64[si];
+    const int ti = d.type_s[si];
+    const int ai = d.atom_of_slot[si];
+    const uint32_t e = d.chunk_j[32 * c + lane];
+    const uint32_t mk = d.chunk_mask[32 * c + lane];
+    const int js = static_cast<int>(e & 0x03FFFFFFu);
+    double4 xj = make_double4(0, 0, 0, 0);
+    int tj = 0;
+    if (mk) {
+        xj = d.xq64[js];
+        tj = d.type_s[js];
+    }
+    if (!MI) {
+        // wrapped positions, the j entry in the image of its code
+        if (ai >= 0) {
+            xi.x -= d.imgx[ai] * L;
+            xi.y -= d.imgy[ai] * L;
+            xi.z -= d.imgz[ai] * L;
+        }
+        if (mk) {
+            const int aj = d.atom_of_slot[js];
+            xj.x -= (d.imgx[aj] - (static_cast<int>((e >> 26) & 3u) - 1)) * L;
+            xj.y -= (d.imgy[aj] - (static_cast<int>((e >> 28) & 3u) - 1)) * L;
+            xj.z -= (d.imgz[aj] - (static_cast<int>((e >> 30) & 3u) - 1)) * L;
+        }
+    }
+    S.xq[lane] = xj;
+    S.tj[lane] = tj;
+    S.js[lane] = js;
+    uint32_t rm = rotated_columns(mk, lane);
+    __syncwarp();
+    const bool has_lj = (R.flags & F_LJ) != 0;
+    const double rl2 = has_lj ? R.rc_lj2 : 0.0, rcc2 = COUL ? R.rc_c2 : 0.0;
+    const double rmax2 = fmax(rl2, rcc2) * (1.0 + 1e-12);
+    const double wl = rl2 * 1e-12, wc = rcc2 * 1e-12;
+    const double keqi = KE * xi.w;
+    double cf[EWALD_N];
+    double us = 0.0;
+    if (COUL) {
+        us = 2.0 / R.rc_c2;
+#pragma unroll
+        for (int k = 0; k < EWALD_N; ++k) cf[k] = d.ewald_poly[EWALD_N * r + k];
+    }
+    const double2* lj = d.lj64 + R.lj_off + ti * R.n_types;
+    double fix = 0, fiy = 0, fiz = 0, fjx = 0, fjy = 0, fjz = 0;
+    double el = 0, ec = 0, vir = 0;
+    const int src_lane = (lane + 1) & 31;
+#pragma unroll 1
+    for (int k = 0; k < 32; ++k) {
+        const int src = (lane + k) & 31;
+        const double4 pj = S.xq[src];
+        double dx = pj.x - xi.x, dy = pj.y - xi.y, dz = pj.z - xi.z;
+        if (MI) {
+            dx = fma(-L, rint(dx * invL), dx);
+            dy = fma(-L, rint(dy * invL), dy);
+            dz = fma(-L, rint(dz * invL), dz);
+        }
+        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+        if ((rm & 1u) && r2 < rmax2) {
+            bool in_l = r2 < rl2, in_c = COUL && r2 < rcc2;
+            if (fabs(r2 - rl2) < wl || (COUL && fabs(r2 - rcc2) < wc)) {
+                const int aj = d.atom_of_slot[S.js[src]];
+                in_l = has_lj && exact_inside(d, ai, aj, L, invL, R.rc_lj2);
+                in_c = COUL && exact_inside(d, ai, aj, L, invL, R.rc_c2);
+            }
+            const double rinv = rsqrt_h(r2);
+            const double ir2 = rinv * rinv;
+            double f = 0.0;
+            if (in_l) {
+                const double2 p = lj[S.tj[src]];
+                const double sr6 = p.y * (ir2 * ir2 * ir2);
+                f = 24.0 * p.x * ir2 * fma(2.0 * sr6, sr6, -sr6);
+                if (ENERGY) el = fma(4.0 * p.x, fma(sr6, sr6, -sr6), el);
+            }
+            if (COUL) {
+                const double u = fma(r2, us, -1.0);
+                const double u2 = u * u;  // even and odd powers: two chains
+                double qe = cf[EWALD_N - 2], qo = cf[EWALD_N - 1];
+#pragma unroll
+                for (int n = EWALD_N - 4; n >= 0; n -= 2) {
+                    qe = fma(qe, u2, cf[n]);
+                    qo = fma(qo, u2, cf[n + 1]);
+                }
+                const double q = fma(qo, u, qe);
+                const double fc = keqi * pj.w * fma(rinv, ir2, -q);
+                f += in_c ? fc : 0.0;
+                if (ENERGY && in_c) ec = fma(keqi * pj.w * rinv, erfc(R.alpha * (r2 * rinv)), ec);
+            }
+            if (ENERGY) vir = fma(f, r2, vir);
+            fix = fma(-f, dx, fix);
+            fiy = fma(-f, dy, fiy);
+            fiz = fma(-f, dz, fiz);
+            fjx = fma(f, dx, fjx);
+            fjy = fma(f, dy, fjy);
+            fjz = fma(f, dz, fjz);
+        }
+        rm >>= 1;
+        fjx = __shfl_sync(FULL, fjx, src_lane);
+        fjy = __shfl_sync(FULL, fjy, src_lane);
+        fjz = __shfl_sync(FULL, fjz, src_lane);
+    }
+    if (ai >= 0) {
+        fix_add(d.fnx + si, to_fix(fix, FSCALE, s));
+        fix_add(d.fny + si, to_fix(fiy, FSCALE, s));
+        fix_add(d.fnz + si, to_fix(fiz, FSCALE, s));
+    }
+    if (mk) {
+        fix_add(d.fnx + js, to_fix(fjx, FSCALE, s));
+        fix_add(d.fny + js, to_fix(fjy, FSCALE, s));
+        fix_add(d.fnz + js, to_fix(fjz, FSCALE, s));
+    }
+    if (ENERGY) {
+        acc.lj += to_fix(el, ESCALE, s);
+        acc.c += to_fix(ec, ESCALE, s);
+        acc.v += to_fix(vir, ESCALE, s);
+    }
+    __syncwarp();
+}
+
+// The energy forms, out of line: their registers do not weigh on the others.
+template <bool COUL, bool MI>
+__device__ __noinline__ void nb_chunk_f64_energy(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
+                                                 ChunkStage64& S, Acc& acc) {
+    nb_chunk_f64<COUL, MI, true>(d, R, s, r, c, lane, S, acc);
+}
+
+// Persistent, chunks claimed as in k_nb_f32 (first chunk without a claim).
+// PHYS tables with real-space Coulomb hold the Ewald coefficients in registers
+// (2 blocks of 256 threads per SM).
 template <bool PHYS>
-__global__ void __launch_bounds__(256) k_nb_f64(Dev d) {
+__global__ void __launch_bounds__(256, 2) k_nb_f64(const __grid_constant__ Dev d) {
     chain_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    __shared__ double4 s_xj[8][32];
-    __shared__ int s_tj[8][32];
-    __shared__ uint32_t s_mk[8][32];
-    const int nw = (gridDim.x * blockDim.x) >> 5;
+    __shared__ ChunkStage64 s_stage[8];
+    const int nw = gridDim.x * 8;
     const int total = d.chunk_prefix[d.n_rep];
     Acc acc{0, 0, 0};
     int cur = -1;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nw) {
+    for (int w = blockIdx.x + gridDim.x * wib; w < total;) {
         const int r = chunk_replica(d.chunk_prefix, d.n_rep, w);
         if (r != cur) {
             flush_acc(d, cur, acc);
             cur = r;
         }
         RepState* s = d.st + r;
-        if (!s->eval) continue;
         const Rep& R = d.rep[r];
-        const int c = R.chunk_begin + (w - d.chunk_prefix[r]);
-        const double L = s->L, invL = s->invL;
-        const int I = d.chunk_itile[c];
-        const int si = 32 * I + lane;
-        const double4 xi = d.xq64[si];
-        const int ti = d.type_s[si];
-        const uint32_t e = d.chunk_j[32 * c + lane];
-        const uint32_t mk = d.chunk_mask[32 * c + lane];
-        const int js = static_cast<int>(e & 0x03FFFFFFu);
-        double4 xj = make_double4(0, 0, 0, 0);
-        int tj = 0;
-        if (mk) {
-            xj = d.xq64[js];
-            tj = d.type_s[js];
-        }
-        s_xj[wib][lane] = xj;
-        s_tj[wib][lane] = tj;
-        s_mk[wib][lane] = mk;
-        __syncwarp();
-        const bool has_lj = (R.flags & F_LJ) != 0;
-        const bool has_c = PHYS && (R.flags & F_COUL_REAL) != 0;
-        const double rl2 = R.rc_lj2, rcc2 = R.rc_c2, alpha = R.alpha;
-        const double2* lj = d.lj64 + R.lj_off + ti * R.n_types;
-        double fix = 0, fiy = 0, fiz = 0, fjx = 0, fjy = 0, fjz = 0;
-        double el = 0, ec = 0, vir = 0;
-        for (int k = 0; k < 32; ++k) {
-            const int src = (lane + k) & 31;
-            const uint32_t m = s_mk[wib][src];
-            if ((m >> lane) & 1u) {
-                const double4 pj = s_xj[wib][src];
-                const double dx = mi_ref(__dsub_rn(pj.x, xi.x), L, invL);
-                const double dy = mi_ref(__dsub_rn(pj.y, xi.y), L, invL);
-                const double dz = mi_ref(__dsub_rn(pj.z, xi.z), L, invL);
-                const double r2 = r2_ref(dx, dy, dz);
-                double f = 0.0;
-                if (has_lj && r2 < rl2) {
-                    // 24 eps (2 sr6^2 - sr6) / r2 and 4 eps (sr6^2 - sr6), reference order
-                    const double2 p = lj[s_tj[wib][src]];
-                    const double r6 = __dmul_rn(__dmul_rn(r2, r2), r2);
-                    const double sr6 = __ddiv_rn(p.y, r6);
-                    f = __ddiv_rn(__dmul_rn(__dmul_rn(24.0, p.x),
-                                            __dsub_rn(__dmul_rn(__dmul_rn(2.0, sr6), sr6), sr6)), r2);
-                    el += __dmul_rn(__dmul_rn(4.0, p.x), __dsub_rn(__dmul_rn(sr6, sr6), sr6));
-                }
-                if (has_c && r2 < rcc2) {
-                    const double qq = KE * xi.w * pj.w;
-                    const double r = sqrt(r2);
-                    const double erfc_ar = erfc(alpha * r);
-                    f += qq * (erfc_ar / (r2 * r) + 2.0 * alpha * exp(-alpha * alpha * r2) /
-                                                        (1.7724538509055160273 * r2));
-                    ec += qq * erfc_ar / r;
-                }
-                vir += f * r2;
-                fix -= f * dx;
-                fiy -= f * dy;
-                fiz -= f * dz;
-                fjx += f * dx;
-                fjy += f * dy;
-                fjz += f * dz;
+        int skip = 0;
+        if (s->eval) {
+            const int c = R.chunk_begin + (w - d.chunk_prefix[r]);
+            const bool coul = PHYS && (R.flags & F_COUL_REAL);
+            const bool mi = 4.0 * R.rc_list2 > s->L * s->L;
+            if (coul && !R.ewald_ok) {
+                nb_chunk_f64_erfc(d, R, s, c, lane, s_stage[wib], acc);
+            } else if (s->want_e) {
+                if (coul && !mi) nb_chunk_f64_energy<PHYS, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+                else if (coul) nb_chunk_f64_energy<PHYS, true>(d, R, s, r, c, lane, s_stage[wib], acc);
+                else if (!mi) nb_chunk_f64_energy<false, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+                else nb_chunk_f64_energy<false, true>(d, R, s, r, c, lane, s_stage[wib], acc);
+            } else if (coul && !mi) {
+                nb_chunk_f64<PHYS, false, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+            } else if (coul) {
+                nb_chunk_f64<PHYS, true, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+            } else if (!mi) {
+                nb_chunk_f64<false, false, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+            } else {
+                nb_chunk_f64<false, true, false>(d, R, s, r, c, lane, s_stage[wib], acc);
             }
-            fjx = __shfl_sync(FULL, fjx, (lane + 1) & 31);
-            fjy = __shfl_sync(FULL, fjy, (lane + 1) & 31);
-            fjz = __shfl_sync(FULL, fjz, (lane + 1) & 31);
+        } else {
+            skip = d.chunk_prefix[r + 1] - nw;  // past this replica's chunks
         }
-        if (d.atom_of_slot[si] >= 0) {
-            fix_add(d.fnx + si, to_fix(fix, FSCALE, s));
-            fix_add(d.fny + si, to_fix(fiy, FSCALE, s));
-            fix_add(d.fnz + si, to_fix(fiz, FSCALE, s));
+        if (total <= nw) break;  // every chunk is some warp's first
+        if (lane == 0) {
+            if (skip > 0) atomicMax(d.nb_work, skip);
+            w = nw + atomicAdd(d.nb_work, 1);
         }
-        if (mk) {
-            fix_add(d.fnx + js, to_fix(fjx, FSCALE, s));
-            fix_add(d.fny + js, to_fix(fjy, FSCALE, s));
-            fix_add(d.fnz + js, to_fix(fjz, FSCALE, s));
-        }
-        acc.lj += to_fix(el, ESCALE, s);
-        acc.c += to_fix(ec, ESCALE, s);
-        acc.v += to_fix(vir, ESCALE, s);
-        __syncwarp();
+        w = __shfl_sync(FULL, w, 0);
     }
     flush_acc(d, cur, acc);
 }
@@ -827,8 +1026,8 @@ void configure_nonbonded_kernels() {
 void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_per_sm, int form,
                       cudaStream_t st, long long* nlaunch) {
     if (fp64) {
-        if (phys) launch_chained(k_nb_f64<true>, n_sm * 8, 256, st, d);
-        else launch_chained(k_nb_f64<false>, n_sm * 8, 256, st, d);
+        if (phys) launch_chained(k_nb_f64<true>, n_sm * 2, 256, st, d);
+        else launch_chained(k_nb_f64<false>, n_sm * 2, 256, st, d);
     } else {
         const bool ljs = d.n_lj <= LJ_SMEM;
         // a table without real-space Coulomb runs the LJ-only instantiation

@@ -27,6 +27,8 @@ constexpr double ESCALE = 4294967296.0;        // 2^32 per kJ mol^-1 (energies, 
 constexpr double MSCALE = 1099511627776.0;     // 2^40 per e (PME mesh charge)
 constexpr double FMAX = 1.0e9;                 // |F| above this -> BondExplosion status
 
+constexpr int EWALD_N = 24;  // coefficients of the FP64 path's real-space Ewald polynomial
+
 enum RepFlags : int {
     F_LJ = 1,          // Lennard-Jones component present
     F_COUL_REAL = 2,   // real-space Ewald on the shared list (phys)
@@ -53,6 +55,7 @@ struct Rep {
     int flags, profile;
     int thermostat, barostat;
     int pme_K;
+    int ewald_ok;                       // the replica has an Ewald polynomial (Dev::ewald_poly)
     long long mesh_fix_off, mesh_fix_n;  // int64 spread buffer (REF: K*K*2(K/2+1), PHYS: K^3)
     long long mesh_real_off;             // K^3 reals
     long long mesh_cplx_off;             // K*K*(K/2+1) complex
@@ -91,6 +94,7 @@ struct RepState {
     double time;
     long long e_acc[N_EACC];
     long long step, target_step;
+    long long read_step;  // energies are formed at this step too (FP64: the last of a call)
     long long andersen_calls;
     long long list_builds;
     int active;           // advances this step
@@ -201,6 +205,7 @@ struct Dev {
     const double2* lj64;               // (eps, sig^6)
     const float4* lj32;                // (c6, c12, 6 c6, 12 c12), c6 = 4 eps sig^6, c12 = 4 eps sig^12
     int n_lj;                          // entries of the LJ tables (all replicas)
+    const double* ewald_poly;          // [n_rep][EWALD_N] (FP64 path), in 2 r^2 / rc_c^2 - 1
     // PME
     long long* mesh_fix;
     void* mesh_real;

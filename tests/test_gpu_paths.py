@@ -82,3 +82,31 @@ def test_pair_set_several_images_and_exclusions(oracle, n_chains, profile):
         r2 = dd[:, 0] * dd[:, 0] + dd[:, 1] * dd[:, 1] + dd[:, 2] * dd[:, 2]
         want.update((i, int(j)) for j in np.nonzero(r2 < rc * rc)[0] + i + 1)
     assert got == want - ex
+
+
+@pytest.mark.parametrize("alpha", [3.12, 4.2])
+@pytest.mark.parametrize("rc_lj", [1.0, 0.85])
+@pytest.mark.parametrize("n_mol", [110, 429])
+def test_fp64_pair_forms(oracle, n_mol, rc_lj, alpha):
+    """FP64 pair forces: Ewald polynomial (alpha rc 3.12) and erfc() (4.2), equal
+    and different cutoffs, boxes narrower (1.49 nm) and wider (2.34 nm) than
+    twice the list cutoff, with and without energies.  Tolerances: 1e-9 for
+    forces (fixed-point step), 1e-8 for a short trajectory."""
+    box = (n_mol / 33.43) ** (1 / 3)
+    c = W.water_box(n_mol=n_mol, box=box, seed=5, spacing=box / round(box / 0.1)).config()
+    c.lj_cutoff, c.ewald_coeff = rc_lj, alpha
+    eng = _engine(c, "fp64", "phys")
+    f, e = eng.compute_forces()
+    f_o, e_o = oracle.forces(c, "phys")
+    assert rel_rms(f, f_o) < 1e-9
+    oe = oracle.engine(c, "phys")
+    oe.step(5)
+    run = _engine(c, "fp64", "phys")
+    run.run_n(5)
+    assert np.abs(run.positions - oe.get(0)).max() < 1e-8
+    assert rel_rms(run.velocities, oe.get(1)) < 1e-8
+    # energies of the evaluation that ends a call do not change its forces
+    one = _engine(c, "fp64", "phys")
+    for _ in range(5):
+        one.run_n(1)
+    assert np.array_equal(one.positions, run.positions)
