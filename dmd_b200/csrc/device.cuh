@@ -33,9 +33,19 @@ __device__ __forceinline__ double r2_ref(double dx, double dy, double dz) {
 __device__ __forceinline__ void set_status(RepState* s, int flag) { atomicOr(&s->status, flag); }
 
 // Fixed-point conversion with range / NaN detection (the value is clamped so the
-// integer conversion is always defined).
+// integer conversion is always defined).  The scales are powers of two and FMAX
+// is an FP32 value, so an FP32 value is scaled exactly in FP32 and converted
+// from there: the same integer as by way of FP64, without the FP64 pipe.
 template <typename T>
 __device__ __forceinline__ long long to_fix(T v, double scale, RepState* s) {
+    if (sizeof(T) == 4) {
+        float f = static_cast<float>(v);
+        if (!(fabsf(f) < static_cast<float>(FMAX))) {
+            set_status(s, (f != f) ? ST_NAN : ST_RANGE);
+            f = (f != f) ? 0.0f : copysignf(static_cast<float>(FMAX), f);
+        }
+        return __float2ll_rn(f * static_cast<float>(scale));
+    }
     double d = static_cast<double>(v);
     if (!(fabs(d) < FMAX)) {
         set_status(s, (d != d) ? ST_NAN : ST_RANGE);

@@ -747,10 +747,11 @@ int Batch::pack() {
             P.bsp_off = static_cast<int>(n_bsp);
             n_bsp += K;
             P.pme_block_begin = pme_blocks;
-            P.pme_blocks = static_cast<int>((static_cast<long long>(K) * K * (K / 2 + 1) + 255) / 256);
+            P.pme_blocks = static_cast<int>((static_cast<long long>(K) * K * (K / 2 + 1) + 256 * PME_POINTS - 1) / (256 * PME_POINTS));
             pme_blocks += P.pme_blocks;
             P.conv_block_begin = conv_blocks;
-            P.conv_blocks = static_cast<int>((P.mesh_fix_n + 1023) / 1024);
+            P.conv_points = P.mesh_fix_n >= (1 << 20) ? 4096 : 1024;
+            P.conv_blocks = static_cast<int>((P.mesh_fix_n + P.conv_points - 1) / P.conv_points);
             conv_blocks += P.conv_blocks;
             any_pme_ = true;
         }
@@ -852,9 +853,11 @@ int Batch::pack() {
             }
             density_ = vol > 0.0 ? static_cast<double>(n_atoms) / vol : 0.0;
         }
-        d.any_coul = 0;
-        for (int k = 0; k < R; ++k)
+        d.any_coul = d.any_wide = 0;
+        for (int k = 0; k < R; ++k) {
             if (reps_[order_[k]]->rep.flags & F_COUL_REAL) d.any_coul = 1;
+            if (reps_[order_[k]]->rep.n_tiles >= WIDE_TILES) d.any_wide = 1;
+        }
         d.grid_bar = A.alloc<unsigned>(2);
         d.build_prefix = A.alloc<int>(4 * (R + 1));
         if (uses_clusters()) {

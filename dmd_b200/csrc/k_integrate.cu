@@ -637,7 +637,8 @@ __global__ void k_energy_reduce(Dev d) {
 }
 
 // Four block-wide sums at once in a fixed order: lane sums by shuffles, then
-// the block's warps in order by warp 0 (blockDim.x = 256).
+// the block's warps by warp 0 (256 or 512 threads; the warps beyond a
+// replica's summing threads hold zeros, which leave its sums as they are).
 __device__ void block_sum4(double v[4], double (*sh)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = warp_sum_d(v[k]);
@@ -650,7 +651,7 @@ __device__ void block_sum4(double v[4], double (*sh)[4]) {
         for (int k = 0; k < 4; ++k) {
             double x = (lane < nw) ? sh[lane][k] : 0.0;
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
             v[k] = x;
         }
     }
@@ -662,20 +663,28 @@ __device__ void block_sum4(double v[4], double (*sh)[4]) {
 // With `next` the next step of the same launch begins here too (begin_step).
 // In a chained launch only the tile partials come from the kernel before it:
 // the replica's records and the PME partials are loaded before the wait.
-__global__ void k_replica_update(Dev d, int next) {
-    __shared__ double sh[8][4];
+__global__ void __launch_bounds__(512) k_replica_update(Dev d, int next) {
+    __shared__ double sh[16][4];
     const int r = blockIdx.x;
     RepState* s = d.st + r;
     const Rep& R = d.rep[r];
     const bool active = s->active != 0;
+    // Threads that sum: 256, or all 512 of a wide launch for a replica of many
+    // tiles (by its own size, so its sums do not depend on what else is in the
+    // table).  Water 750k, 23,438 tiles and 27,936 PME
+    // partials (now 6,984): 59 -> 12 us.
+    const int nt = R.n_tiles >= WIDE_TILES ? static_cast<int>(blockDim.x) : 256;
+    const bool summing = static_cast<int>(threadIdx.x) < nt;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     RepState st;
     Rep Rr;
     if (active) {
-        if (R.flags & F_PME) {
-            for (int b = threadIdx.x; b < R.pme_blocks; b += blockDim.x) {
-                v[2] += d.pme_part[2 * (R.pme_block_begin + b)];
-                v[3] += d.pme_part[2 * (R.pme_block_begin + b) + 1];
+        if ((R.flags & F_PME) && summing) {
+            const double2* pp = reinterpret_cast<const double2*>(d.pme_part) + R.pme_block_begin;
+            for (int b = threadIdx.x; b < R.pme_blocks; b += nt) {
+                const double2 ev = pp[b];
+                v[2] += ev.x;
+                v[3] += ev.y;
             }
         }
         // one thread uses these: the replica's records copied to registers at
@@ -688,9 +697,12 @@ __global__ void k_replica_update(Dev d, int next) {
     chain_wait();
     if (next && r == 0 && threadIdx.x == 0) reset_counters(d);
     if (!active) return;
-    for (int t = R.tile_begin + threadIdx.x; t < R.tile_begin + R.n_tiles; t += blockDim.x) {
-        v[0] += d.tile_ke[t];
-        v[1] += d.tile_vir[t];
+    if (summing) {
+#pragma unroll 4
+        for (int t = R.tile_begin + threadIdx.x; t < R.tile_begin + R.n_tiles; t += nt) {
+            v[0] += d.tile_ke[t];
+            v[1] += d.tile_vir[t];
+        }
     }
     block_sum4(v, sh);
     if (threadIdx.x != 0) return;
@@ -868,7 +880,7 @@ void launch_rattle(const Dev& d, cudaStream_t st, long long* n) {
     *n += 2;
 }
 void launch_replica_update(const Dev& d, bool next, cudaStream_t st, long long* n) {
-    launch_chained(k_replica_update, d.n_rep, 256, st, d, next ? 1 : 0);
+    launch_chained(k_replica_update, d.n_rep, d.any_wide ? 512 : 256, st, d, next ? 1 : 0);
     ++*n;
 }
 void launch_apply_scale(const Dev& d, bool, cudaStream_t st, long long* n) {

@@ -402,7 +402,8 @@ __global__ void __launch_bounds__(256, PHYS ? 3 : 4) k_nb_f32(Dev d) {
                     }
                 }
             }
-            if (total <= nw) break;  // every chunk is some warp's first
+            // every chunk is some warp's first, or no later replica is this kernel's
+            if (total <= nw || next >= d.n_rep) break;
             if (lane == 0) {
                 const int skip = d.chunk_prefix[next] - nw;
                 if (skip > 0) atomicMax(counter, skip);

@@ -27,6 +27,8 @@ constexpr double ESCALE = 4294967296.0;        // 2^32 per kJ mol^-1 (energies, 
 constexpr double MSCALE = 1099511627776.0;     // 2^40 per e (PME mesh charge)
 constexpr double FMAX = 1.0e9;                 // |F| above this -> BondExplosion status
 
+constexpr int WIDE_TILES = 4096;  // replicas of at least this many tiles are reduced by 512 threads
+constexpr int PME_POINTS = 4;  // mesh points per thread of the influence kernel (256 threads per block)
 constexpr int EWALD_N = 24;  // coefficients of the FP64 path's real-space Ewald polynomial
 
 enum RepFlags : int {
@@ -61,7 +63,8 @@ struct Rep {
     long long mesh_cplx_off;             // K*K*(K/2+1) complex
     int bsp_off;                         // K doubles: B-spline factor per mesh index
     int pme_block_begin, pme_blocks;     // influence-kernel blocks
-    int conv_block_begin, conv_blocks;   // convert-kernel blocks (1,024 mesh points each)
+    int conv_block_begin, conv_blocks;   // convert-kernel blocks
+    int conv_points;                     // mesh points per convert block (1,024 or 4,096)
     double rc_lj, rc_c, rc_list;
     double rc_lj2, rc_c2, rc_list2, half_skin2;
     double alpha;
@@ -172,6 +175,7 @@ struct Dev {
     int* nb_work;                      // pair-kernel chunk counter (reset per evaluation)
     int* nb_work_mi;                   // the same for the narrow-box pair kernel
     int mi_split;                      // narrow-box replicas go to their own pair kernel
+    int any_wide;                      // some replica has at least WIDE_TILES tiles
     int any_coul;                      // some replica has real-space Coulomb (F_COUL_REAL)
     int* build_work;                   // list-build i-tile counter (reset per rebuild)
     int* build_prefix;                 // [3][n_rep + 1] prefixes of the rebuilding replicas'

@@ -110,3 +110,31 @@ def test_fp64_pair_forms(oracle, n_mol, rc_lj, alpha):
     for _ in range(5):
         one.run_n(1)
     assert np.array_equal(one.positions, run.positions)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_mol,spacing", [(130, 0.2), (400, 0.105), (400, 0.022)])
+def test_pme_mesh_sizes(oracle, n_mol, spacing, precision):
+    """SPME on meshes of 8^3 (one block), 22^3 (a ragged last block) and 104^3 (the
+    four-groups-per-thread conversion, above 2^20 points): forces and the
+    reciprocal energy against the oracle.  Tolerances: the single-point ones."""
+    box = (n_mol / 33.43) ** (1 / 3)
+    c = W.water_box(n_mol=n_mol, box=box, seed=9, spacing=spacing).config()
+    f, e = _engine(c, precision, "phys").compute_forces()
+    f_o, e_o = oracle.forces(c, "phys")
+    assert rel_rms(f, f_o) < {"fp64": 1e-9, "mixed": 1e-5}[precision]
+
+
+def test_energies_of_mixed_blocks(oracle):
+    """Bonded energies where a block's terms belong to several replicas: a batch
+    of small decane melts gives each the energies it has alone, bit for bit."""
+    from dmd_b200.batch import Batch
+    cfgs = [W.decane_melt(n, 20 + n).config() for n in (9, 12, 10, 17, 9)]
+    b = Batch(precision="mixed", profile="phys")
+    slots = [b.admit(c, 3) for c in cfgs]
+    b.step(3)
+    for c, k in zip(cfgs, slots):
+        eng = _engine(c, "mixed", "phys")
+        eng.run_n(3)
+        assert list(b.scalars(k).e_terms) == list(eng.scalars().e_terms)
+        assert np.array_equal(b.positions(k), eng.positions)
