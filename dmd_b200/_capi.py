@@ -132,6 +132,8 @@ def lib() -> C.CDLL:
         "dmdgpu_run": (C.c_int, [vp]),
         "dmdgpu_get_state": (C.c_int, [vp, C.c_int32, _dp, _dp, _dp]),
         "dmdgpu_set_state": (C.c_int, [vp, C.c_int32, _dp, _dp, _dp]),
+        "dmdgpu_get_state_rows": (C.c_int, [vp, C.c_int32, _dp]),
+        "dmdgpu_set_state_rows": (C.c_int, [vp, C.c_int32, _dp]),
         "dmdgpu_get_scalars": (C.c_int, [vp, C.POINTER(dmdgpu_scalars)]),
         "dmdgpu_compute_forces": (C.c_int, [vp, _dp, _dp, _dp, _dp]),
         "dmdgpu_component_compute": (C.c_int, [vp, C.c_int32, _dp, _dp, _dp, C.c_double,
@@ -155,6 +157,7 @@ def lib() -> C.CDLL:
         "dmdgpu_batch_step_timed": (C.c_int, [vp, C.c_int32, C.c_int64, C.POINTER(dmdgpu_timing)]),
         "dmdgpu_batch_poll": (C.c_int, [vp, _ip, C.c_int32, C.POINTER(C.c_int32)]),
         "dmdgpu_batch_get_state": (C.c_int, [vp, C.c_int32, C.c_int32, _dp, _dp, _dp]),
+        "dmdgpu_batch_get_state_rows": (C.c_int, [vp, C.c_int32, C.c_int32, _dp]),
         "dmdgpu_batch_get_scalars": (C.c_int, [vp, C.c_int32, C.POINTER(dmdgpu_scalars)]),
         "dmdgpu_batch_release": (C.c_int, [vp, C.c_int32]),
         "dmdgpu_batch_used_bytes": (C.c_int64, [vp]),

@@ -95,11 +95,9 @@ class Batch:
         return buf[:min(n.value, cap)].tolist()
 
     def _state(self, slot, which):
-        n = self._n[slot]
-        x, y, z = np.empty(n), np.empty(n), np.empty(n)
-        self._check(self._lib.dmdgpu_batch_get_state(self._h, int(slot), which, _capi.dptr(x),
-                                                     _capi.dptr(y), _capi.dptr(z)))
-        return np.stack([x, y, z], axis=1)
+        rows = np.empty((self._n[slot], 3))
+        self._check(self._lib.dmdgpu_batch_get_state_rows(self._h, int(slot), which, _capi.dptr(rows)))
+        return rows
 
     def positions(self, slot: int) -> np.ndarray:
         return self._state(slot, 0)

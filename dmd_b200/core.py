@@ -211,12 +211,9 @@ class Engine:
         self._check(self._lib.dmdgpu_step(self._h, int(steps)))
 
     def _state(self, which):
-        x = np.empty(self._n)
-        y = np.empty(self._n)
-        z = np.empty(self._n)
-        self._check(self._lib.dmdgpu_get_state(self._h, which, _capi.dptr(x), _capi.dptr(y),
-                                               _capi.dptr(z)))
-        return np.stack([x, y, z], axis=1)
+        rows = np.empty((self._n, 3))
+        self._check(self._lib.dmdgpu_get_state_rows(self._h, which, _capi.dptr(rows)))
+        return rows
 
     @property
     def positions(self):
@@ -261,23 +258,26 @@ class Engine:
         s = self.scalars()
         return {k: s.e_terms[i] for i, k in enumerate(_capi.E_TERMS)}
 
+    def _set_state(self, which, rows):
+        rows = np.asarray(rows, dtype=np.float64)
+        if rows.shape == (self._n, 3):
+            rows = np.ascontiguousarray(rows)
+            self._check(self._lib.dmdgpu_set_state_rows(self._h, which, _capi.dptr(rows)))
+            return
+        x, y, z = (np.ascontiguousarray(rows[:, k]) for k in range(3))
+        self._check(self._lib.dmdgpu_set_state(self._h, which, _capi.dptr(x), _capi.dptr(y), _capi.dptr(z)))
+
     def set_positions(self, pos):
-        pos = np.asarray(pos, dtype=np.float64)
-        x, y, z = (np.ascontiguousarray(pos[:, k]) for k in range(3))
-        self._check(self._lib.dmdgpu_set_state(self._h, 0, _capi.dptr(x), _capi.dptr(y), _capi.dptr(z)))
+        self._set_state(0, pos)
 
     def set_velocities(self, vel):
-        vel = np.asarray(vel, dtype=np.float64)
-        x, y, z = (np.ascontiguousarray(vel[:, k]) for k in range(3))
-        self._check(self._lib.dmdgpu_set_state(self._h, 1, _capi.dptr(x), _capi.dptr(y), _capi.dptr(z)))
+        self._set_state(1, vel)
 
     def compute_forces(self):
         """Single-point forces (N x 3) and energy terms at the current positions."""
-        fx, fy, fz = np.empty(self._n), np.empty(self._n), np.empty(self._n)
         e = np.zeros(len(_capi.E_TERMS))
-        self._check(self._lib.dmdgpu_compute_forces(self._h, _capi.dptr(fx), _capi.dptr(fy),
-                                                    _capi.dptr(fz), _capi.dptr(e)))
-        return np.stack([fx, fy, fz], axis=1), dict(zip(_capi.E_TERMS, e))
+        self._check(self._lib.dmdgpu_compute_forces(self._h, None, None, None, _capi.dptr(e)))
+        return self._state(2), dict(zip(_capi.E_TERMS, e))
 
     def component_compute(self, component: int, pos, box, forces=None, energy=0.0):
         """ForceComponent::compute: accumulate one component's forces/energy."""

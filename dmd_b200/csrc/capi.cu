@@ -177,6 +177,18 @@ int dmdgpu_set_state(dmdgpu_ctx* c, int32_t which, const double* x, const double
     return rc ? ctx_fail(c, rc) : DMDGPU_OK;
 }
 
+int dmdgpu_get_state_rows(dmdgpu_ctx* c, int32_t which, double* rows) {
+    if (!c || !c->b || !rows) return DMDGPU_ERR_INVALID;
+    int rc = c->b->get_state_rows(c->slot, which, rows);
+    return rc ? ctx_fail(c, rc) : DMDGPU_OK;
+}
+
+int dmdgpu_set_state_rows(dmdgpu_ctx* c, int32_t which, const double* rows) {
+    if (!c || !c->b || !rows) return DMDGPU_ERR_INVALID;
+    int rc = c->b->set_state_rows(c->slot, which, rows);
+    return rc ? ctx_fail(c, rc) : DMDGPU_OK;
+}
+
 int dmdgpu_get_scalars(dmdgpu_ctx* c, dmdgpu_scalars* out) {
     if (!c || !c->b || !out) return DMDGPU_ERR_INVALID;
     int rc = c->b->get_scalars(c->slot, out);
@@ -368,6 +380,13 @@ int dmdgpu_batch_poll(dmdgpu_batch* b, int32_t* slots, int32_t cap, int32_t* n_d
 int dmdgpu_batch_get_state(dmdgpu_batch* b, int32_t slot, int32_t which, double* x, double* y, double* z) {
     if (!b || !b->b || !x || !y || !z) return DMDGPU_ERR_INVALID;
     int rc = b->b->get_state(slot, which, x, y, z);
+    if (rc) b->err = b->b->error();
+    return rc;
+}
+
+int dmdgpu_batch_get_state_rows(dmdgpu_batch* b, int32_t slot, int32_t which, double* rows) {
+    if (!b || !b->b || !rows) return DMDGPU_ERR_INVALID;
+    int rc = b->b->get_state_rows(slot, which, rows);
     if (rc) b->err = b->b->error();
     return rc;
 }

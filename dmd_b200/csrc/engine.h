@@ -101,6 +101,7 @@ struct PinnedStaging {
     size_t blk = 0, off = 0;
     void* put(const void* src, size_t bytes);
     void reset() { blk = off = 0; }
+    std::pair<char*, size_t> block();  // the first block, whole (between table rebuilds)
     void trim(size_t keep);       // frees the later blocks beyond `keep` bytes
     ~PinnedStaging() { trim(0); }
 };
@@ -124,6 +125,8 @@ class Batch {
     int compute_forces(int slot, double* fx, double* fy, double* fz, double* e_terms);
     int get_state(int slot, int which, double* x, double* y, double* z);
     int set_state(int slot, int which, const double* x, const double* y, const double* z);
+    int get_state_rows(int slot, int which, double* rows);
+    int set_state_rows(int slot, int which, const double* rows);
     int get_scalars(int slot, dmdgpu_scalars* out);
     int pair_list(int slot, int32_t* pi, int32_t* pj, long long cap, long long* count);
     int save_checkpoint(int slot, const char* path);
@@ -192,6 +195,9 @@ class Batch {
     std::map<int, std::pair<cufftHandle, cufftHandle>> plans_;
     cudaGraphExec_t graph_ = nullptr;       // one step
     cudaGraphExec_t graph_many_ = nullptr;  // kManySteps steps (tables that keep running)
+    int copy_out(int slot, int which, double* const out[3], bool rows);
+    int copy_in(int slot, int which, const double* const in[3], bool rows);
+    cudaEvent_t ev_state_[2] = {};          // pieces of a state being copied out
     bool joined_ = false;                   // the last evaluation joined other streams
     long long steps_run_ = 0;               // steps launched from graph_ or graph_many_
     int capture_steps(int n, cudaGraphExec_t* out);

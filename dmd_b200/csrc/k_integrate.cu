@@ -827,6 +827,59 @@ __global__ void k_frame_snapshot(Dev d, int r, double* out) {
     o[5 * n + i] = lam == 1.0 ? d.vz[a] : __dmul_rn(d.vz[a], lam);
 }
 
+// n atoms from a0 on into host memory that the device can write (pinned): which
+// 0 positions, 1 velocities with the pending thermostat scale applied as
+// k_finalize_v would (no state is changed), 2 forces; rows: [n][3], otherwise
+// three arrays `stride` apart.
+__global__ void k_export_state(Dev d, int a0, int n, int which, int rows, long long stride, double* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int a = a0 + i;
+    double v[3];
+    if (which == 0) {
+        v[0] = d.x[a];
+        v[1] = d.y[a];
+        v[2] = d.z[a];
+    } else if (which == 1) {
+        const double lam = d.st[d.atom_rep[a]].vscale;
+        v[0] = lam == 1.0 ? d.vx[a] : __dmul_rn(d.vx[a], lam);
+        v[1] = lam == 1.0 ? d.vy[a] : __dmul_rn(d.vy[a], lam);
+        v[2] = lam == 1.0 ? d.vz[a] : __dmul_rn(d.vz[a], lam);
+    } else {
+        const int s = d.slot_of_atom[a];
+        v[0] = from_fix(d.fbx[a] + d.fnx[s], FSCALE);
+        v[1] = from_fix(d.fby[a] + d.fny[s], FSCALE);
+        v[2] = from_fix(d.fbz[a] + d.fnz[s], FSCALE);
+    }
+    for (int c = 0; c < 3; ++c) out[rows ? 3LL * i + c : c * stride + i] = v[c];
+}
+
+// The reverse for replica r's positions (0: its list and forces are then due)
+// and velocities (1: any pending thermostat scale is dropped with the old ones).
+__global__ void k_import_state(Dev d, int r, int a0, int n, int which, int rows, long long stride, const double* in) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        if (which == 0) {
+            d.st[r].rebuild = 1;
+            d.st[r].have_forces = 0;
+        } else {
+            d.st[r].vscale = 1.0;
+        }
+    }
+    if (i >= n) return;
+    double v[3];
+    for (int c = 0; c < 3; ++c) v[c] = in[rows ? 3LL * i + c : c * stride + i];
+    const int a = a0 + i;
+    double* x = which == 0 ? d.x : d.vx;
+    double* y = which == 0 ? d.y : d.vy;
+    double* z = which == 0 ? d.z : d.vz;
+    x[a] = v[0];
+    y[a] = v[1];
+    z[a] = v[2];
+}
+
+__global__ void k_request_rebuild(Dev d, int r) { d.st[r].rebuild = 1; }
+
 __global__ void k_finalize_reset(Dev d) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < d.n_rep) d.st[r].vscale = 1.0;
@@ -894,6 +947,20 @@ void launch_finalize_velocities(const Dev& d, cudaStream_t st, long long* n) {
 }
 void launch_frame_snapshot(const Dev& d, int r, int n_atoms, double* out, cudaStream_t st, long long* n) {
     k_frame_snapshot<<<(n_atoms + 255) / 256, 256, 0, st>>>(d, r, out);
+    ++*n;
+}
+void launch_export_state(const Dev& d, int a0, int n, int which, bool rows, long long stride, double* out,
+                         cudaStream_t st, long long* nl) {
+    k_export_state<<<(n + 255) / 256, 256, 0, st>>>(d, a0, n, which, rows ? 1 : 0, stride, out);
+    ++*nl;
+}
+void launch_import_state(const Dev& d, int r, int a0, int n, int which, bool rows, long long stride, const double* in,
+                         cudaStream_t st, long long* nl) {
+    k_import_state<<<(n + 255) / 256, 256, 0, st>>>(d, r, a0, n, which, rows ? 1 : 0, stride, in);
+    ++*nl;
+}
+void launch_request_rebuild(const Dev& d, int r, cudaStream_t st, long long* n) {
+    k_request_rebuild<<<1, 1, 0, st>>>(d, r);
     ++*n;
 }
 void launch_energy_reduce(const Dev& d, cudaStream_t st, long long* n) {

@@ -74,6 +74,14 @@ void launch_rattle(const Dev& d, cudaStream_t st, long long* nlaunch);
 void launch_replica_update(const Dev& d, bool next, cudaStream_t st, long long* nlaunch);
 void launch_apply_scale(const Dev& d, bool fp64, cudaStream_t st, long long* nlaunch);
 void launch_finalize_velocities(const Dev& d, cudaStream_t st, long long* nlaunch);
+// atoms a0 .. a0 + n - 1 (one replica's) to and from pinned host memory: which 0
+// positions, 1 velocities, 2 forces (export only); rows: [n][3], otherwise three
+// arrays `stride` doubles apart
+void launch_export_state(const Dev& d, int a0, int n, int which, bool rows, long long stride, double* out,
+                         cudaStream_t st, long long* nlaunch);
+void launch_import_state(const Dev& d, int r, int a0, int n, int which, bool rows, long long stride, const double* in,
+                         cudaStream_t st, long long* nlaunch);
+void launch_request_rebuild(const Dev& d, int r, cudaStream_t st, long long* nlaunch);
 void launch_energy_reduce(const Dev& d, cudaStream_t st, long long* nlaunch);
 // replica r's frame (step, time, box, positions, velocities) into `out`
 // (3 + 6 n_atoms doubles), state unchanged

@@ -168,6 +168,9 @@ int dmdgpu_get_state(dmdgpu_ctx *ctx, int32_t which, double *x, double *y, doubl
 /* Overwrite positions (which=0) or velocities (which=1). */
 int dmdgpu_set_state(dmdgpu_ctx *ctx, int32_t which, const double *x, const double *y,
                      const double *z);
+/* The same as one array of n_atoms rows (x, y, z). */
+int dmdgpu_get_state_rows(dmdgpu_ctx *ctx, int32_t which, double *rows);
+int dmdgpu_set_state_rows(dmdgpu_ctx *ctx, int32_t which, const double *rows);
 int dmdgpu_get_scalars(dmdgpu_ctx *ctx, dmdgpu_scalars *out);
 
 /* Single-point evaluation of every component at the current positions
@@ -333,6 +336,7 @@ int dmdgpu_batch_step_timed(dmdgpu_batch *b, int32_t n_steps, int64_t l2_flush_b
 int dmdgpu_batch_poll(dmdgpu_batch *b, int32_t *slots, int32_t cap, int32_t *n_done);
 int dmdgpu_batch_get_state(dmdgpu_batch *b, int32_t slot, int32_t which, double *x, double *y,
                            double *z);
+int dmdgpu_batch_get_state_rows(dmdgpu_batch *b, int32_t slot, int32_t which, double *rows);
 int dmdgpu_batch_get_scalars(dmdgpu_batch *b, int32_t slot, dmdgpu_scalars *out);
 int dmdgpu_batch_release(dmdgpu_batch *b, int32_t slot);
 int64_t dmdgpu_batch_used_bytes(dmdgpu_batch *b);

@@ -138,3 +138,35 @@ def test_energies_of_mixed_blocks(oracle):
         eng.run_n(3)
         assert list(b.scalars(k).e_terms) == list(eng.scalars().e_terms)
         assert np.array_equal(b.positions(k), eng.positions)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [64, 65536, 65537, 140001])
+def test_state_rows_and_arrays(n, precision):
+    """State copies of one piece, exactly one, just above and several: rows,
+    separate arrays and what was set agree bit for bit, and reading velocities
+    leaves a pending thermostat scale as it is."""
+    import ctypes
+    from dmd_b200 import _capi
+    c = W.lj_fluid(n, 0.7, 1.0, 3).config()
+    c.thermostat.type, c.thermostat.temperature = "berendsen", 90.0
+    eng = _engine(c, precision, "phys")
+    rng = np.random.default_rng(1)
+    x = np.stack([c.pos_x, c.pos_y, c.pos_z], 1)
+    v = rng.normal(size=(n, 3))
+    eng.set_positions(x)
+    eng.set_velocities(v)
+    assert np.array_equal(eng.positions, x) and np.array_equal(eng.velocities, v)
+    eng.run_n(2)
+    for which, rows in ((0, eng.positions), (1, eng.velocities), (2, eng.forces)):
+        a = [np.empty(n) for _ in range(3)]
+        assert eng._lib.dmdgpu_get_state(eng._h, which, *(_capi.dptr(k) for k in a)) == 0
+        assert np.array_equal(np.stack(a, 1), rows)
+    other = _engine(c, precision, "phys")
+    other.set_positions(x)
+    other.set_velocities(np.hstack([v, v])[:, :4])  # more columns: the first three count
+    other.run_n(1)
+    other.velocities
+    other.run_n(1)
+    assert np.array_equal(other.velocities, eng.velocities)
+    assert eng._lib.dmdgpu_get_state_rows(eng._h, 3, _capi.dptr(np.empty((n, 3)))) == 4  # DMDGPU_ERR_PARM
