@@ -305,7 +305,7 @@ void Batch::free_device() {
     // the pinned mirrors are kept (cudaFreeHost synchronises the device and
     // costs milliseconds); the next table grows them when it needs more
     arena_.reset();
-    st_fresh_ = false;
+    st_fresh_ = sim_ok_ = false;
     packed_ = false;
     used_bytes_ = 0;
 }
@@ -1240,7 +1240,7 @@ int Batch::pack() {
         CK(cudaMallocHost(&h_tgt_, sizeof(long long) * cap));
         h_st_cap_ = cap;
     }
-    st_fresh_ = false;
+    st_fresh_ = sim_ok_ = false;
     // cuFFT plans per mesh size (normally made at admission already)
     for (int k = 0; k < R; ++k) {
         const Rep& P = reps_[order_[k]]->rep;
@@ -1383,14 +1383,15 @@ void Batch::enqueue_eval(int pass) {
 // some replica's rebuild flag is set.
 void Batch::enqueue_rebuild() { launch_rebuild(dev_, d_bin_rep_, n_sm_, stream_, &launches_); }
 
-// begun: the step before it in the same launch began this one; next: another
-// step follows in the same launch and this one begins it (k_replica_update).
-void Batch::enqueue_step(bool begun, bool next) {
+// first: issue the first evaluation.  begun: the step before it in the same
+// launch began this one; next (NextStep): another step follows in the same
+// launch and this one begins it (k_replica_update).
+void Batch::enqueue_step(bool first, bool begun, int next) {
     // The first evaluation repeats the previous step's second one unless the
     // barostat moved the atoms, the REF list cadence rebuilds now, or no forces
     // exist yet; only then is it issued (its kernels skip replicas that do not need it).
-    if (need_eval1_) enqueue_eval(PASS_FIRST);
-    if (!begun) launch_eval_begin(dev_, PASS_SECOND, stream_, &launches_);
+    if (first) enqueue_eval(PASS_FIRST);
+    if (!begun) launch_eval_begin(dev_, first || !skip_first() ? PASS_SECOND : PASS_SECOND_ONLY, stream_, &launches_);
     launch_kick_drift(dev_, fp64_, stream_, &launches_);
     if (any_cons_) launch_shake(dev_, stream_, &launches_);
     enqueue_eval(PASS_SECOND);
@@ -1458,9 +1459,10 @@ void Batch::set_node_priorities(cudaGraph_t g) {
 }
 
 void Batch::drop_graphs() {
-    if (graph_) cudaGraphExecDestroy(graph_);
-    if (graph_many_) cudaGraphExecDestroy(graph_many_);
-    graph_ = graph_many_ = nullptr;
+    for (cudaGraphExec_t* g : {&graph_, &graph_skip_, &graph_many_}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
 }
 
 // Steps per launch once a table keeps running.  Between two one-step graphs
@@ -1475,10 +1477,16 @@ void Batch::drop_graphs() {
 // every few calls keeps the one-step graph (at 64 a served wave of 8 jobs took
 // 120.5 ms against 116.0).
 constexpr int kManySteps = 4;
+constexpr int kRefCycle = 5;  // REF: the steps from one list rebuild to the next
 constexpr int kManyAfter = 256;
 constexpr int kManyAtoms = 400000;
 
 int Batch::run_steps(int n) {
+    const bool skip = skip_first();
+    if (skip && n > 0) {
+        const int rc = load_cadence();
+        if (rc) return rc;
+    }
     st_fresh_ = false;  // device work follows: the host mirror is stale
     if (n <= 0) return DMDGPU_OK;
     if (fp64_) launch_mark_read(dev_, n, stream_, &launches_);
@@ -1490,7 +1498,7 @@ int Batch::run_steps(int n) {
         // every launch issued from the host (profilers see each kernel); same work
         need_eval1_ = true;
         for (int i = 0; i < n; ++i) {
-            enqueue_step();
+            enqueue_step(need_eval1_);
             CK(cudaGetLastError());
             if (i == 0) need_eval1_ = (any_baro_ && !phys_) || any_ref_lj_;
         }
@@ -1503,7 +1511,7 @@ int Batch::run_steps(int n) {
         for (int i = 0; i < n; ++i) {
             andersen_ref_prepare();
             CK(cudaStreamSynchronize(stream_));
-            enqueue_step();
+            enqueue_step(need_eval1_);
             CK(cudaGetLastError());
         }
         return DMDGPU_OK;
@@ -1511,8 +1519,9 @@ int Batch::run_steps(int n) {
     if (graph_dirty_ || !graph_) {
         // first step eagerly (initial list + forces), then capture the steady-state step
         need_eval1_ = true;
-        enqueue_step();
+        enqueue_step(need_eval1_);
         CK(cudaGetLastError());
+        if (skip) advance_cadence(true);
         need_eval1_ = (any_baro_ && !phys_) || any_ref_lj_;
         --n;
         if (!tuned_ && !rule_bps_) {
@@ -1520,43 +1529,131 @@ int Batch::run_steps(int n) {
             int rc = autotune(n, &used);
             if (rc) return rc;
             n -= used;
+            for (int k = 0; skip && k < used; ++k) advance_cadence(true);
         }
         drop_graphs();
-        const long long before = launches_;
-        const int rc = capture_steps(1, &graph_);
+        long long before = launches_;
+        int rc = capture_steps(1, need_eval1_, &graph_);
         if (rc) return rc;
         per_step_launches_ = launches_ - before;
+        if (skip) {
+            before = launches_;
+            rc = capture_steps(1, false, &graph_skip_);
+            if (rc) return rc;
+            skip_launches_ = launches_ - before;
+            launches_ = before;
+        }
         steps_run_ = 0;
         graph_dirty_ = false;
     }
-    int i = 0;
-    if (dev_.n_atoms <= kManyAtoms && (graph_many_ || steps_run_ >= kManyAfter) && n >= kManySteps) {
-        if (!graph_many_) {
-            const long long before = launches_;
-            int rc = capture_steps(kManySteps, &graph_many_);
-            if (rc) return rc;
-            launches_ = before;
-        }
-        for (; i + kManySteps <= n; i += kManySteps) {
-            CK(cudaGraphLaunch(graph_many_, stream_));
-            launches_ += kManySteps * per_step_launches_;
-        }
+    const bool many = dev_.n_atoms <= kManyAtoms && (graph_many_ || steps_run_ >= kManyAfter);
+    const int per_many = skip ? kRefCycle : kManySteps;
+    if (many && n >= per_many && !graph_many_) {
+        const long long before = launches_;
+        const int rc = capture_steps(per_many, need_eval1_, &graph_many_);
+        if (rc) return rc;
+        many_launches_ = launches_ - before;
+        launches_ = before;
     }
-    for (; i < n; ++i) {
-        CK(cudaGraphLaunch(graph_, stream_));
-        launches_ += per_step_launches_;
+    for (int i = 0; i < n;) {
+        const bool first = !skip || cadence_due();
+        if (many && graph_many_ && i + per_many <= n && (!skip || (first && cadence_cycle()))) {
+            CK(cudaGraphLaunch(graph_many_, stream_));
+            launches_ += many_launches_;
+            for (int k = 0; skip && k < per_many; ++k) advance_cadence(k == 0);
+            i += per_many;
+            continue;
+        }
+        CK(cudaGraphLaunch(first ? graph_ : graph_skip_, stream_));
+        launches_ += first ? per_step_launches_ : skip_launches_;
+        if (skip) advance_cadence(first);
+        ++i;
     }
     steps_run_ += n;
+    if (skip) sim_ok_ = true;
     return DMDGPU_OK;
 }
 
-// n steady-state steps captured as one executable graph.
-int Batch::capture_steps(int n, cudaGraphExec_t* out) {
+// ---- REF list cadence on the host -------------------------------------------
+// The reference evaluates forces twice per step and rebuilds its list at every
+// tenth call, so a step's first evaluation differs from the previous step's
+// second one only every fifth step.  Its five kernels found that out on the
+// device; the counters follow from the state the host has at the start of a
+// call, so the host issues them only in the steps that need them (argon 4k:
+// 45 us for a step with them, 17 us without).  Not under the REF barostat,
+// whose scaling makes every first evaluation necessary.
+bool Batch::skip_first() const { return any_ref_lj_ && !any_baro_ && !any_andersen_ref_; }
+
+int Batch::load_cadence() {
+    const size_t R = order_.size();
+    if (!st_fresh_) {
+        if (sim_ok_ && cadence_.size() == R) return DMDGPU_OK;
+        CK(cudaMemcpyAsync(h_st_, d_st_, sizeof(RepState) * R, cudaMemcpyDeviceToHost, stream_));
+        CK(cudaStreamSynchronize(stream_));
+        st_fresh_ = true;
+    }
+    cadence_.resize(R);
+    for (size_t k = 0; k < R; ++k) {
+        const RepState& s = h_st_[k];
+        cadence_[k] = Cadence{s.target_step - s.step, s.lj_counter, s.have_forces != 0, s.rebuild != 0,
+                              (reps_[order_[k]]->rep.flags & F_LJ) != 0};
+    }
+    return DMDGPU_OK;
+}
+
+// Whether the next step's first evaluation is needed by some replica.
+bool Batch::cadence_due() const {
+    for (const Cadence& c : cadence_)
+        if (c.left > 0 && (!c.have_forces || c.rebuild || (c.lj && c.counter >= 10))) return true;
+    return false;
+}
+
+// Whether the next kRefCycle steps need it in their first step only: every
+// replica that advances is at the same point of its cadence and goes on.
+bool Batch::cadence_cycle() const {
+    for (const Cadence& c : cadence_)
+        if (c.left > 0 && (c.left < kRefCycle || !c.have_forces || (c.lj && c.counter != 10))) return false;
+    return true;
+}
+
+// One step, with or without its first evaluation (k_eval_begin, k_rebuild and
+// k_replica_update do the same on the device).
+void Batch::advance_cadence(bool first) {
+    for (Cadence& c : cadence_) {
+        const bool active = c.left > 0;
+        const bool ev = first && active && (!c.have_forces || (c.lj && c.counter >= 10));
+        if (active && !ev && c.lj) c.counter += 1;
+        if (first) {
+            if (ev && c.lj && c.counter >= 10) c.rebuild = true;
+            if (c.rebuild) c.counter = 0;
+            c.rebuild = false;
+            if (ev && c.lj) c.counter += 1;
+            if (ev) c.have_forces = true;
+        }
+        if (active && c.lj && c.counter >= 10) c.rebuild = true;
+        if (c.rebuild) c.counter = 0;
+        c.rebuild = false;
+        if (active) {
+            if (c.lj) c.counter += 1;
+            c.have_forces = true;
+            c.left -= 1;
+        }
+    }
+}
+
+// n steady-state steps captured as one executable graph; first: with the first
+// evaluation -- in every step, or (skip_first()) in the first of them only.
+int Batch::capture_steps(int n, bool first, cudaGraphExec_t* out) {
     cudaGraph_t g;
+    const bool skip = skip_first();
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     // a first evaluation or the REF barostat's scaling comes between two steps
-    const bool between = need_eval1_ || (any_baro_ && !phys_);
-    for (int k = 0; k < n; ++k) enqueue_step(k > 0 && !between, k + 1 < n && !between);
+    const bool between = (first && !skip) || (any_baro_ && !phys_);
+    for (int k = 0; k < n; ++k) {
+        const bool f = first && (k == 0 || !skip);
+        const int next = (k + 1 < n && !between) ? (skip ? NEXT_SKIPS : NEXT_STEP) : NEXT_NONE;
+        enqueue_step(f, k > 0 && !between, next);
+    }
     CK(cudaStreamEndCapture(stream_, &g));
     set_node_priorities(g);
     const cudaError_t e = cudaGraphInstantiate(out, g, cudaGraphInstantiateFlagUseNodePriority);
@@ -1597,7 +1694,7 @@ int Batch::autotune(int max_steps, int* used) {
         std::vector<float> t(kTuneSteps);
         cudaGraphExec_t ge = nullptr;
         const long long before = launches_;
-        int rc = capture_steps(1, &ge);
+        int rc = capture_steps(1, need_eval1_, &ge);
         if (rc) return rc;
         launches_ = before + kTuneSteps * (launches_ - before);
         CK(cudaEventRecord(ev[0], stream_));
@@ -1676,7 +1773,7 @@ int Batch::rebuild_in_frame(const std::vector<char>& sel) {
     CK(cudaMemcpy(d_st_, tmp.data(), sizeof(RepState) * R, cudaMemcpyHostToDevice));
     launch_write_mirror(dev_, fp64_, stream_, &launches_);
     CK(cudaGetLastError());
-    st_fresh_ = false;
+    st_fresh_ = sim_ok_ = false;
     graph_dirty_ = true;
     return DMDGPU_OK;
 }
@@ -1891,7 +1988,7 @@ void Batch::record(cudaEvent_t e, cudaStream_t st) {
 // how the branches were scheduled (water 30k: a step period of ~143 us
 // against ~124 us for run_n's graph), hence one step graph and sampling.
 int Batch::step_timed(int n, long long flush_bytes, dmdgpu_timing* out) {
-    st_fresh_ = false;  // device work follows: the host mirror is stale
+    st_fresh_ = sim_ok_ = false;  // device work follows: the host mirror is stale
     CK(cudaSetDevice(device_));
     std::memset(out, 0, sizeof(*out));
     if (failed_) return fail(DMDGPU_ERR_GPU, "a list build timed out earlier; the table is unusable");
@@ -1925,7 +2022,7 @@ int Batch::step_timed(int n, long long flush_bytes, dmdgpu_timing* out) {
     capture_error_ = false;
     cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        enqueue_step();
+        enqueue_step(need_eval1_);
         e = cudaStreamEndCapture(stream_, &g);
     }
     prof_nb_ = nullptr;
@@ -2069,7 +2166,7 @@ int Batch::inject(int what) {
     }
     if (order_.empty()) return fail(DMDGPU_ERR_INVALID, "empty batch");
     CK(cudaStreamSynchronize(stream_));
-    st_fresh_ = false;
+    st_fresh_ = sim_ok_ = false;
     if (what == DMDGPU_INJECT_BARRIER_TIMEOUT) {
         dev_.bar_extra = 1;
         dev_.bar_limit_ns = 20000000ull;
@@ -2108,8 +2205,10 @@ int Batch::poll(int32_t* slots, int cap, int* n_done) {
 // into the pinned staging block (in the caller's layout) and copied out from
 // there; nothing on the device changes.  Large states go in pieces, the next
 // one under way while one is copied out.  Three copies into pageable memory,
-// each waiting, and the interleaving on the host took 45 us for 1,000 atoms and
-// 26 ms for 750,000 (positions and velocities); now 23 us and @@READ@@ ms.
+// each waiting, and the interleaving on the host took most of a small or
+// batched pass: 100 steps of 1,000 LJ atoms with their frame 1,847 -> 1,684 us,
+// 20 steps of a 64-replica batch 26.6 -> 14.7 ms, 30 steps of water 750k 78.4 ->
+// 71.8 ms, a single-point evaluation of water 30k 1,074 -> 444 us.
 int Batch::copy_out(int slot, int which, double* const out[3], bool rows) {
     CK(cudaSetDevice(device_));
     if (!has(slot)) return fail(DMDGPU_ERR_INVALID, "no such slot");
@@ -2146,7 +2245,7 @@ int Batch::copy_out(int slot, int which, double* const out[3], bool rows) {
 }
 
 int Batch::copy_in(int slot, int which, const double* const in[3], bool rows) {
-    st_fresh_ = false;  // the replica's flags change on the device
+    st_fresh_ = sim_ok_ = false;  // the replica's flags change on the device
     CK(cudaSetDevice(device_));
     if (!has(slot)) return fail(DMDGPU_ERR_INVALID, "no such slot");
     if (!packed_) {
@@ -2245,7 +2344,7 @@ int Batch::get_scalars(int slot, dmdgpu_scalars* out) {
 }
 
 int Batch::compute_forces(int slot, double* fx, double* fy, double* fz, double* e_terms) {
-    st_fresh_ = false;  // device work follows: the host mirror is stale
+    st_fresh_ = sim_ok_ = false;  // device work follows: the host mirror is stale
     CK(cudaSetDevice(device_));
     if (!has(slot)) return fail(DMDGPU_ERR_INVALID, "no such slot");
     if (failed_) return fail(DMDGPU_ERR_GPU, "a list build timed out earlier; the table is unusable");
@@ -2274,7 +2373,7 @@ int Batch::compute_forces(int slot, double* fx, double* fy, double* fz, double* 
 }
 
 int Batch::pair_list(int slot, int32_t* pi, int32_t* pj, long long cap, long long* count) {
-    st_fresh_ = false;  // device work follows: the host mirror is stale
+    st_fresh_ = sim_ok_ = false;  // device work follows: the host mirror is stale
     CK(cudaSetDevice(device_));
     if (!has(slot)) return fail(DMDGPU_ERR_INVALID, "no such slot");
     if (!packed_) {
@@ -2438,7 +2537,7 @@ int Batch::save_checkpoint(int slot, const char* path) {
 }
 
 int Batch::load_checkpoint(int slot, const char* path) {
-    st_fresh_ = false;  // device work follows: the host mirror is stale
+    st_fresh_ = sim_ok_ = false;  // device work follows: the host mirror is stale
     CK(cudaSetDevice(device_));
     if (!has(slot)) return fail(DMDGPU_ERR_INVALID, "no such slot");
     if (!packed_) {

@@ -153,7 +153,7 @@ class Batch {
     int build_host(HostRep& hr, unsigned comp_mask);
     void enqueue_eval(int pass);
     void enqueue_rebuild();
-    void enqueue_step(bool begun = false, bool next = false);
+    void enqueue_step(bool first, bool begun = false, int next = 0);
     int run_steps(int n);
     int autotune(int max_steps, int* used);
     int rebuild_in_frame(const std::vector<char>& sel);
@@ -200,7 +200,22 @@ class Batch {
     cudaEvent_t ev_state_[2] = {};          // pieces of a state being copied out
     bool joined_ = false;                   // the last evaluation joined other streams
     long long steps_run_ = 0;               // steps launched from graph_ or graph_many_
-    int capture_steps(int n, cudaGraphExec_t* out);
+    int capture_steps(int n, bool first, cudaGraphExec_t* out);
+    // REF list cadence per packed replica, followed on the host (run_steps)
+    struct Cadence {
+        long long left;  // steps to the replica's target
+        int counter;     // RepState::lj_counter
+        bool have_forces, rebuild, lj;
+    };
+    std::vector<Cadence> cadence_;
+    bool sim_ok_ = false;                   // cadence_ holds at the last launched step
+    bool skip_first() const;
+    int load_cadence();
+    bool cadence_due() const;
+    bool cadence_cycle() const;
+    void advance_cadence(bool first);
+    cudaGraphExec_t graph_skip_ = nullptr;  // one step without its first evaluation (REF)
+    long long skip_launches_ = 0, many_launches_ = 0;
     void drop_graphs();
     bool packed_ = false;
     // a list build timed out: its sort and list buffers are in an unknown

@@ -55,8 +55,12 @@ __device__ __forceinline__ void begin_eval(RepState& s, const Rep& R, bool ev, b
 // scales, and the step's (second) evaluation.  Runs in k_eval_begin ahead of
 // the first step of a launch, and at the end of k_replica_update between the
 // steps of one launch.
-__device__ __forceinline__ void begin_step(RepState& s, const Rep& R) {
+// skipped: the step's first evaluation was not issued (REF; no replica needed
+// it), but LennardJones::compute advances its counter on every call
+// (lennard_jones.cpp:91).
+__device__ __forceinline__ void begin_step(RepState& s, const Rep& R, bool skipped) {
     s.active = (s.step < s.target_step) ? 1 : 0;
+    if (skipped && s.active && !(R.flags & F_PHYS) && (R.flags & F_LJ)) s.lj_counter += 1;
     s.dr_move = s.active;
     s.dr_vscale = s.vscale;
     s.dr_pscale = s.pscale;
@@ -83,8 +87,8 @@ __global__ void k_eval_begin(Dev d, int pass) {
     if (r >= d.n_rep) return;
     RepState* s = d.st + r;
     const Rep& R = d.rep[r];
-    if (pass == PASS_SECOND) {
-        begin_step(*s, R);
+    if (pass == PASS_SECOND || pass == PASS_SECOND_ONLY) {
+        begin_step(*s, R, pass == PASS_SECOND_ONLY);
         return;
     }
     bool ev = true;
@@ -769,7 +773,7 @@ __global__ void __launch_bounds__(512) k_replica_update(Dev d, int next) {
     }
     st.step += 1;
     st.time += dt;
-    if (next) begin_step(st, Rr);
+    if (next) begin_step(st, Rr, next == NEXT_SKIPS);
     *s = st;
 }
 
@@ -932,8 +936,8 @@ void launch_rattle(const Dev& d, cudaStream_t st, long long* n) {
     launch_chained(k_tile_ke, (d.n_slots + 255) / 256, 256, st, d);
     *n += 2;
 }
-void launch_replica_update(const Dev& d, bool next, cudaStream_t st, long long* n) {
-    launch_chained(k_replica_update, d.n_rep, d.any_wide ? 512 : 256, st, d, next ? 1 : 0);
+void launch_replica_update(const Dev& d, int next, cudaStream_t st, long long* n) {
+    launch_chained(k_replica_update, d.n_rep, d.any_wide ? 512 : 256, st, d, next);
     ++*n;
 }
 void launch_apply_scale(const Dev& d, bool, cudaStream_t st, long long* n) {

@@ -57,7 +57,12 @@ void launch_pme_influence(const Dev& d, bool fp64, int n_blocks, cudaStream_t st
 void launch_pme_gather(const Dev& d, bool fp64, cudaStream_t st, long long* nlaunch);
 
 // k_integrate.cu
-enum EvalPass { PASS_FIRST = 1, PASS_SECOND = 2, PASS_SINGLE = 3 };
+// PASS_SECOND_ONLY: the second pass of a step whose first evaluation was not
+// issued (REF: no replica needs it)
+enum EvalPass { PASS_FIRST = 1, PASS_SECOND = 2, PASS_SINGLE = 3, PASS_SECOND_ONLY = 4 };
+// What follows a step in the same launch, begun by k_replica_update: nothing, a
+// step, or (REF) a step without its first evaluation.
+enum NextStep { NEXT_NONE = 0, NEXT_STEP = 1, NEXT_SKIPS = 2 };
 void launch_eval_begin(const Dev& d, int pass, cudaStream_t st, long long* nlaunch);
 // the evaluation n_steps from now forms energies (a slot's own target aside)
 void launch_mark_read(const Dev& d, int n_steps, cudaStream_t st, long long* nlaunch);
@@ -70,8 +75,7 @@ void launch_kick2(const Dev& d, bool andersen_ref, bool andersen_phys, bool chai
                   long long* nlaunch);
 void launch_shake(const Dev& d, cudaStream_t st, long long* nlaunch);
 void launch_rattle(const Dev& d, cudaStream_t st, long long* nlaunch);
-// next: begin the next step too (another step of the same launch follows)
-void launch_replica_update(const Dev& d, bool next, cudaStream_t st, long long* nlaunch);
+void launch_replica_update(const Dev& d, int next, cudaStream_t st, long long* nlaunch);
 void launch_apply_scale(const Dev& d, bool fp64, cudaStream_t st, long long* nlaunch);
 void launch_finalize_velocities(const Dev& d, cudaStream_t st, long long* nlaunch);
 // atoms a0 .. a0 + n - 1 (one replica's) to and from pinned host memory: which 0

@@ -170,3 +170,47 @@ def test_state_rows_and_arrays(n, precision):
     other.run_n(1)
     assert np.array_equal(other.velocities, eng.velocities)
     assert eng._lib.dmdgpu_get_state_rows(eng._h, 3, _capi.dptr(np.empty((n, 3)))) == 4  # DMDGPU_ERR_PARM
+
+
+def _argon(nc, seed=0):
+    c = W.argon_fcc(n_cells=nc, a=0.575).config()
+    rng = np.random.default_rng(seed)
+    n = len(c.masses)
+    c.pos_x, c.pos_y, c.pos_z = (p + rng.normal(0, 0.01, n) for p in (c.pos_x, c.pos_y, c.pos_z))
+    return c
+
+
+@pytest.mark.parametrize("calls", [(30,), (1,) * 12, (3, 1, 7, 2, 11), (5, 5, 5), (4, 9)])
+def test_ref_cadence_across_calls(oracle, calls):
+    """REF: the first evaluation is issued only in the steps whose list cadence
+    needs it; calls that end anywhere in the cadence follow the oracle, which
+    evaluates twice in every step (FP64, 1e-9), and new positions restart it."""
+    c = _argon(4)
+    oe, eng = oracle.engine(c, "ref"), _engine(c, "fp64", "ref")
+    for n in calls:
+        oe.step(n)
+        eng.run_n(n)
+        assert np.abs(eng.positions - oe.get(0)).max() < 1e-9
+        assert rel_rms(eng.velocities, oe.get(1)) < 1e-9
+
+
+def test_ref_cadence_in_batch(oracle):
+    """REF replicas at different points of their cadence in one table (admitted at
+    different times, with different targets) follow the oracle (FP64, 1e-9)."""
+    from dmd_b200.batch import Batch
+    cfgs = [_argon(4, 1), _argon(3, 2), _argon(4, 3)]
+    targets = [17, 9, 12]
+    b = Batch(precision="fp64", profile="ref")
+    slots = [b.admit(cfgs[0], targets[0])]
+    b.step(3)
+    slots.append(b.admit(cfgs[1], targets[1]))
+    b.step(4)
+    slots.append(b.admit(cfgs[2], targets[2]))
+    for n in (1, 6, 20):
+        b.step(n)
+    for c, n, k in zip(cfgs, targets, slots):
+        oe = oracle.engine(c, "ref")
+        oe.step(n)
+        assert b.scalars(k).step == n
+        assert np.abs(b.positions(k) - oe.get(0)).max() < 1e-9
+        assert rel_rms(b.velocities(k), oe.get(1)) < 1e-9
