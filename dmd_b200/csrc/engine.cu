@@ -194,9 +194,8 @@ static bool ewald_polynomial(double alpha, double rc, double* out) {
 // ---------------------------------------------------------------------------
 // Autotuner cache: the pair kernel's launch shape chosen for a kind of batch,
 // shared by every batch of the process (the serving loop repacks often).
-// Key: device, precision, whether a PME chain runs beside the pair kernel, and
-// the batch's atom count in powers of four (a served stream's table changes
-// size with every admission; nearby sizes share a shape).
+// Key: device, precision, whether a PME chain runs beside the pair kernel, the
+// forced form, the table's atom count and density.
 namespace {
 struct TuneKey {
     int device, fp64, pme, bucket, forced, dens;
@@ -213,17 +212,17 @@ std::mutex g_tune_mu;
 std::map<TuneKey, TuneChoice> g_tune;
 constexpr size_t kStatePiece = 65536;       // atoms of a state copied through the staging block at a time
 constexpr int kTuneSteps = 6;               // timed steps per candidate
-// (4 blocks per SM: the LJ-only chunk kernel only, which a table without
-// real-space Coulomb runs; for the others the launch takes 3)
-constexpr TuneChoice kTuneCand[] = {{NB_CLUSTER8, 1}, {NB_CLUSTER8, 2}, {NB_CHUNK32, 2}, {NB_CHUNK32, 3},
-                                    {NB_CHUNK32, 4}};
+// (only tables with a PME chain are tuned; 4 blocks per SM, for LJ-only tables,
+// come from the rule)
+constexpr TuneChoice kTuneCand[] = {{NB_CLUSTER8, 1}, {NB_CLUSTER8, 2}, {NB_CHUNK32, 1}, {NB_CHUNK32, 2},
+                                    {NB_CHUNK32, 3}};
 
 // forced: the caller's dmdgpu_options.nb_form (0: the default form)
-// bucket: atom count in powers of four; dens: the table's atoms per nm^3 in
-// powers of two (LJ fluids ~16-22, water ~100)
+// bucket: atom count in powers of the square root of two (what runs beside the
+// pair kernel for how long changes within a factor of two); dens: the table's
+// atoms per nm^3 in powers of two (LJ fluids ~16-22, water ~100)
 TuneKey tune_key(int device, bool fp64, bool pme, long long n_atoms, int forced, double density) {
-    int b = 0;
-    while ((1LL << (2 * b + 2)) <= n_atoms) ++b;
+    const int b = n_atoms > 0 ? static_cast<int>(std::floor(2.0 * std::log2(static_cast<double>(n_atoms)))) : 0;
     const int dens = density > 0.0 ? static_cast<int>(std::floor(std::log2(density))) : 0;
     return TuneKey{device, fp64 ? 1 : 0, pme ? 1 : 0, b, forced, dens};
 }
@@ -1271,9 +1270,10 @@ int Batch::pack() {
         // of 33.0 us at 2 blocks, 37.7 at 4; water 30k 126 us at 2 against 142
         // at 3.  Above 400,000 atoms every kernel fills the GPU by itself and
         // the chain gains nothing from running beside (750k: 2.79 ms at 2
-        // blocks, 2.74 at 3).  A table with a PME chain measures the other
-        // shapes too (autotune).
-        rule_bps_ = !fp64_ && !any_pme_ && nb_form_ == NB_CHUNK32;
+        // blocks, 2.74 at 3).  A single system with a PME chain measures the
+        // other shapes too (autotune); a batch, whose table changes with every
+        // admission, keeps the rule's.
+        rule_bps_ = !fp64_ && (!any_pme_ || R > 1) && nb_form_ == NB_CHUNK32;
         tuned_ = fp64_ || it != g_tune.end();
         if (nb_form_ == NB_CLUSTER8) {
             nb_blocks_per_sm_ = 2;
@@ -1282,7 +1282,12 @@ int Batch::pack() {
             for (int k = 0; k < R; ++k) chunks += n_chunks_built_[k];
             const long long per_block = 8LL * n_sm_;
             const bool beside = dev_.n_bonds + dev_.n_excl > 0 || any_pme_;
-            const int most = (dev_.any_coul ? 3 : 4) - (beside && dev_.n_atoms < 400000 ? 1 : 0);
+            int most = (dev_.any_coul ? 3 : 4) - (beside && dev_.n_atoms < 400000 ? 1 : 0);
+            // A short list beside a PME chain: the chain's kernels are then the
+            // longer branch, and one pair block per SM slows them least while it
+            // still ends first (water 9k, 6,858 chunks: 3.25 ms per 50 steps at 1
+            // block, 3.57 at 2; water 30k, 22,800 chunks: 6.79 against 5.20).
+            if (any_pme_ && chunks <= 6 * per_block) most = 1;
             nb_blocks_per_sm_ =
                 static_cast<int>(std::min<long long>(most, std::max<long long>(1, (chunks + per_block - 1) / per_block)));
         }
