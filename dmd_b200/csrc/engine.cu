@@ -875,7 +875,7 @@ int Batch::pack() {
             if (reps_[order_[k]]->rep.flags & F_COUL_REAL) d.any_coul = 1;
             if (reps_[order_[k]]->rep.n_tiles >= WIDE_TILES) d.any_wide = 1;
         }
-        d.grid_bar = A.alloc<unsigned>(2);
+        d.grid_bar = A.alloc<unsigned>(3);
         d.build_prefix = A.alloc<int>(4 * (R + 1));
         if (uses_clusters()) {
             d.tile_nch = A.alloc<int>(n_tiles);

@@ -180,7 +180,7 @@ struct Dev {
     int* build_work;                   // list-build i-tile counter (reset per rebuild)
     int* build_prefix;                 // [3][n_rep + 1] prefixes of the rebuilding replicas'
                                        // atoms, sort cells and tiles
-    unsigned* grid_bar;                // [2] rebuild grid barrier: arrivals, generation
+    unsigned* grid_bar;                // [3] rebuild grid barrier: arrivals, generation; finished blocks
     unsigned long long bar_limit_ns;   // a barrier wait gives up after this long (0: one second)
     unsigned bar_extra;                // arrivals a barrier needs beyond the grid's blocks (0;
                                        // only the failure-path test hook sets it)

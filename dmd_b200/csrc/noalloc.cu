@@ -57,7 +57,7 @@ struct Layout {
 
 constexpr size_t scratch_bytes() {
     size_t b = 0;
-    b += up256(sizeof(Rep)) + up256(sizeof(RepState)) + up256(8 * sizeof(int));  // rep, state, prefix
+    b += up256(sizeof(Rep)) + up256(sizeof(RepState)) + up256(15 * sizeof(int));  // rep, state, prefix
     b += 3 * up256(NA * sizeof(int));              // imgx/y/z
     b += 3 * up256(NA * sizeof(double));           // xr/yr/zr
     b += 3 * up256(NA * sizeof(int));              // atom_rep, slot_of_atom, atom_bin
@@ -180,12 +180,12 @@ extern "C" int dmdgpu_nonbonded_noalloc(const dmdgpu_nb_params* p, const double*
     d.n_bins = nbins;
     Rep* d_rep = reinterpret_cast<Rep*>(at(sizeof(Rep)));
     RepState* d_st = reinterpret_cast<RepState*>(at(sizeof(RepState)));
-    d.chunk_prefix = reinterpret_cast<int*>(at(8 * sizeof(int)));
-    d.build_prefix = d.chunk_prefix + 8;  // [3][2]: words 8..13 of the 256-byte block
+    d.chunk_prefix = reinterpret_cast<int*>(at(15 * sizeof(int)));
+    d.build_prefix = d.chunk_prefix + 9;  // [3][2]: words 9..14 of the 256-byte block
     d.nb_work = d.chunk_prefix + 4;  // zeroed with the prefix below
     d.nb_work_mi = d.chunk_prefix + 3;  // words 0, 1: the chunk prefix of the one replica
     d.build_work = d.chunk_prefix + 5;
-    d.grid_bar = reinterpret_cast<unsigned*>(d.chunk_prefix + 6);  // [2]: words 6, 7
+    d.grid_bar = reinterpret_cast<unsigned*>(d.chunk_prefix + 6);  // [3]: words 6..8
     d.rep = d_rep;
     d.st = d_st;
     d.x = const_cast<double*>(d_x);
@@ -327,7 +327,7 @@ extern "C" int dmdgpu_nonbonded_noalloc(const dmdgpu_nb_params* p, const double*
                 ok(cudaMemsetAsync(d.fnx, 0, sizeof(long long) * 32 * ntiles, st)) &&
                 ok(cudaMemsetAsync(d.fny, 0, sizeof(long long) * 32 * ntiles, st)) &&
                 ok(cudaMemsetAsync(d.fnz, 0, sizeof(long long) * 32 * ntiles, st)) &&
-                ok(cudaMemsetAsync(d.chunk_prefix, 0, 8 * sizeof(int), st));
+                ok(cudaMemsetAsync(d.chunk_prefix, 0, 9 * sizeof(int), st));
     if (!good) return DMDGPU_ERR_GPU;
     long long nl = 0;
     // every launch is checked as soon as it is issued
