@@ -291,6 +291,10 @@ Batch::~Batch() {
     if (ev_join_) cudaEventDestroy(ev_join_);
     if (ev_join_b_) cudaEventDestroy(ev_join_b_);
     if (bond_stream_) cudaStreamDestroy(bond_stream_);
+    for (int l = 0; l < kFftLanes; ++l) {
+        if (ev_fft_[l]) cudaEventDestroy(ev_fft_[l]);
+        if (fft_stream_[l]) cudaStreamDestroy(fft_stream_[l]);
+    }
     if (aux_stream_) cudaStreamDestroy(aux_stream_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -631,6 +635,47 @@ int Batch::ensure_plans(int K) {
     cufftSetStream(b, aux_stream_);
     plans_[K] = {f, b};
     return DMDGPU_OK;
+}
+
+// The replicas' transforms are short kernels in a row (about 3 us each, six per
+// replica): replicas of different mesh sizes run theirs on up to kFftLanes
+// streams side by side.  Those of one size share a plan and its work area, so
+// they share a stream.
+int Batch::assign_fft_lanes() {
+    std::map<int, int> lane;  // mesh size -> lane, in table order
+    for (int k : order_) {
+        const Rep& P = reps_[k]->rep;
+        if ((P.flags & F_PME) && !lane.count(P.pme_K)) {
+            const int n = static_cast<int>(lane.size());
+            lane[P.pme_K] = n % kFftLanes;
+        }
+    }
+    fft_lanes_ = std::min<int>(kFftLanes, static_cast<int>(lane.size()));
+    for (int l = 1; l < fft_lanes_; ++l) {
+        if (fft_stream_[l]) continue;
+        CK(cudaStreamCreateWithPriority(&fft_stream_[l], cudaStreamNonBlocking, prio_hi_));
+        CK(cudaEventCreateWithFlags(&ev_fft_[l], cudaEventDisableTiming));
+        if (!ev_fft_[0]) CK(cudaEventCreateWithFlags(&ev_fft_[0], cudaEventDisableTiming));
+    }
+    for (auto& kv : lane) {
+        const cudaStream_t st = kv.second ? fft_stream_[kv.second] : aux_stream_;
+        cufftSetStream(plans_[kv.first].first, st);
+        cufftSetStream(plans_[kv.first].second, st);
+    }
+    return DMDGPU_OK;
+}
+
+void Batch::fft_fork() {
+    if (fft_lanes_ < 2) return;
+    cudaEventRecord(ev_fft_[0], aux_stream_);
+    for (int l = 1; l < fft_lanes_; ++l) cudaStreamWaitEvent(fft_stream_[l], ev_fft_[0], 0);
+}
+
+void Batch::fft_join() {
+    for (int l = 1; l < fft_lanes_; ++l) {
+        cudaEventRecord(ev_fft_[l], fft_stream_[l]);
+        cudaStreamWaitEvent(aux_stream_, ev_fft_[l], 0);
+    }
 }
 
 int Batch::release(int slot) {
@@ -1248,6 +1293,10 @@ int Batch::pack() {
             if (rc) return rc;
         }
     }
+    {
+        const int rc = assign_fft_lanes();
+        if (rc) return rc;
+    }
     for (int k : order_) reps_[k]->on_device = true;
     {
         // every replica's list, built in the frame of its last build (a new
@@ -1337,6 +1386,7 @@ void Batch::enqueue_eval(int pass) {
         }
         launch_pme_spread(d, fp64_, aux_stream_, &launches_);
         launch_pme_convert(d, fp64_, n_conv_blocks_, aux_stream_, &launches_);
+        fft_fork();
         for (int k : order_) {
             const Rep& P = reps_[k]->rep;
             if (!(P.flags & F_PME)) continue;
@@ -1349,7 +1399,9 @@ void Batch::enqueue_eval(int pass) {
                              static_cast<cufftComplex*>(d.mesh_cplx) + P.mesh_cplx_off);
             }
         }
+        fft_join();
         launch_pme_influence(d, fp64_, n_pme_blocks_, aux_stream_, &launches_);
+        fft_fork();
         for (int k : order_) {
             const Rep& P = reps_[k]->rep;
             if (!(P.flags & F_PME)) continue;
@@ -1362,6 +1414,7 @@ void Batch::enqueue_eval(int pass) {
                              static_cast<float*>(d.mesh_real) + P.mesh_real_off);
             }
         }
+        fft_join();
         launch_pme_gather(d, fp64_, aux_stream_, &launches_);
         if (prof_pme_) {
             e1 = next_event();

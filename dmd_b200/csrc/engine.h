@@ -170,6 +170,14 @@ class Batch {
     cudaStream_t stream_ = nullptr;
     // bonded + PME run on aux_stream_, forked from and joined back to stream_
     cudaStream_t aux_stream_ = nullptr;
+    // transforms of different mesh sizes side by side (lane 0: aux_stream_)
+    static constexpr int kFftLanes = 4;
+    int fft_lanes_ = 1;
+    cudaStream_t fft_stream_[kFftLanes] = {};
+    cudaEvent_t ev_fft_[kFftLanes] = {};
+    int assign_fft_lanes();
+    void fft_fork();
+    void fft_join();
     // bonded terms on a third stream, beside both
     cudaStream_t bond_stream_ = nullptr;
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr, ev_join_b_ = nullptr;
