@@ -330,7 +330,7 @@ __global__ void k_kick2(Dev d, int andersen_ref, int andersen_phys) {
 // operands, so the sweeps are bit for bit those of the general path, which
 // re-reads every operand from global memory in each of its dependent steps.
 // The sweeps are one dependent FP64 chain per thread, so their latency is the
-// kernel's time: 522 molecules, 43.4 -> 19.3 us (SHAKE) and 60.6 -> 19.0 us
+// kernel's time: 522 molecules, 43.4 -> 14.3 us (SHAKE) and 60.6 -> 12.8 us
 // (RATTLE) against the general path.
 __device__ __forceinline__ bool is_triangle(const Dev& d, int c0, int c1, int3& at) {
     if (c1 - c0 != 3) return false;
@@ -339,12 +339,24 @@ __device__ __forceinline__ bool is_triangle(const Dev& d, int c0, int c1, int3& 
     return v.x == u.x && w.x == u.y && w.y == v.y;
 }
 
-// dx - round(dx * inv) * L; a displacement inside half a box (the usual case)
-// has round() = 0 and is returned as it is, which is the same value.
-__device__ __forceinline__ double wrap_ref(double dx, double L, double inv) {
-    const double q = __dmul_rn(dx, inv);
-    if (!(fabs(q) >= 0.5)) return dx;
-    return __dsub_rn(dx, __dmul_rn(round(q), L));
+// d - round(d * inv) * L along each axis; a displacement inside half a box (the
+// usual case) has round() = 0 and is returned as it is, which is the same value.
+__device__ __forceinline__ void wrap_ref(double& dx, double& dy, double& dz, double L, double inv) {
+    const double m = fmax(fmax(fabs(dx), fabs(dy)), fabs(dz));
+    if (!(__dmul_rn(m, inv) >= 0.5)) return;
+    dx = __dsub_rn(dx, __dmul_rn(round(__dmul_rn(dx, inv)), L));
+    dy = __dsub_rn(dy, __dmul_rn(round(__dmul_rn(dy, inv)), L));
+    dz = __dsub_rn(dz, __dmul_rn(round(__dmul_rn(dz, inv)), L));
+}
+
+// a / b with y = 1 / b (correctly rounded): Markstein's division (P. Markstein,
+// IBM J. Res. Dev. 34, 1990), the quotient estimate a y and one correction by
+// its exact remainder.  The correctly rounded quotient, in three dependent
+// operations instead of a full division in every sweep (b does not change
+// between sweeps).
+__device__ __forceinline__ double div_known(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
 }
 
 __device__ __forceinline__ double dot_ref(double ax, double ay, double az, double bx, double by, double bz) {
@@ -354,24 +366,25 @@ __device__ __forceinline__ double dot_ref(double ax, double ay, double az, doubl
 // SHAKE sweeps of one triangle (see k_shake).
 __device__ __forceinline__ void shake_triangle(double (&x)[3], double (&y)[3], double (&z)[3], const double (&w)[3],
                                                const double (&dist)[3], double L, double inv, double tol) {
-    double d2[3], den[3];
+    double d2[3], den[3], rden[3];
     bool ok[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const int a = c == 2 ? 1 : 0, b = c == 0 ? 1 : 2;
         d2[c] = __dmul_rn(dist[c], dist[c]);
         den[c] = __dmul_rn(__dmul_rn(2.0, d2[c]), __dadd_rn(w[a], w[b]));
+        rden[c] = 1.0 / den[c];
     }
     for (int it = 0; it < 100; ++it) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int a = c == 2 ? 1 : 0, b = c == 0 ? 1 : 2;
-            const double dx = wrap_ref(__dsub_rn(x[b], x[a]), L, inv), dy = wrap_ref(__dsub_rn(y[b], y[a]), L, inv),
-                         dz = wrap_ref(__dsub_rn(z[b], z[a]), L, inv);
+            double dx = __dsub_rn(x[b], x[a]), dy = __dsub_rn(y[b], y[a]), dz = __dsub_rn(z[b], z[a]);
+            wrap_ref(dx, dy, dz, L, inv);
             const double err = __dsub_rn(dot_ref(dx, dy, dz, dx, dy, dz), d2[c]);
             ok[c] = !(fabs(err) >= tol);
             if (fabs(err) > tol) {
-                const double lam = err / den[c];
+                const double lam = div_known(err, den[c], rden[c]);
                 const double lx = __dmul_rn(lam, dx), ly = __dmul_rn(lam, dy), lz = __dmul_rn(lam, dz);
                 x[a] = __dadd_rn(x[a], __dmul_rn(lx, w[a]));
                 y[a] = __dadd_rn(y[a], __dmul_rn(ly, w[a]));
@@ -385,20 +398,31 @@ __device__ __forceinline__ void shake_triangle(double (&x)[3], double (&y)[3], d
     }
 }
 
-// RATTLE sweeps of one triangle (see k_rattle): the bond vectors do not change.
-__device__ __forceinline__ void rattle_triangle(const double (&x)[3], const double (&y)[3], const double (&z)[3],
-                                                double (&vx)[3], double (&vy)[3], double (&vz)[3],
-                                                const double (&w)[3], double L, double inv, double tol) {
-    double dx[3], dy[3], dz[3], den[3];
-    bool ok[3];
+// RATTLE of one triangle (see k_rattle): its bond vectors and denominators do
+// not change between sweeps.
+struct TriangleBonds {
+    double dx[3], dy[3], dz[3], den[3], rden[3];
+    __device__ __forceinline__ void set(const double (&x)[3], const double (&y)[3], const double (&z)[3],
+                                        const double (&w)[3], double L, double inv) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const int a = c == 2 ? 1 : 0, b = c == 0 ? 1 : 2;
-        dx[c] = wrap_ref(__dsub_rn(x[b], x[a]), L, inv);
-        dy[c] = wrap_ref(__dsub_rn(y[b], y[a]), L, inv);
-        dz[c] = wrap_ref(__dsub_rn(z[b], z[a]), L, inv);
-        den[c] = __dmul_rn(dot_ref(dx[c], dy[c], dz[c], dx[c], dy[c], dz[c]), __dadd_rn(w[a], w[b]));
+        for (int c = 0; c < 3; ++c) {
+            const int a = c == 2 ? 1 : 0, b = c == 0 ? 1 : 2;
+            dx[c] = __dsub_rn(x[b], x[a]);
+            dy[c] = __dsub_rn(y[b], y[a]);
+            dz[c] = __dsub_rn(z[b], z[a]);
+            wrap_ref(dx[c], dy[c], dz[c], L, inv);
+            den[c] = __dmul_rn(dot_ref(dx[c], dy[c], dz[c], dx[c], dy[c], dz[c]), __dadd_rn(w[a], w[b]));
+            rden[c] = 1.0 / den[c];
+        }
     }
+};
+
+__device__ __forceinline__ void rattle_triangle(const TriangleBonds& tb, double (&vx)[3], double (&vy)[3],
+                                                double (&vz)[3], const double (&w)[3], double tol) {
+    const double(&dx)[3] = tb.dx;
+    const double(&dy)[3] = tb.dy;
+    const double(&dz)[3] = tb.dz;
+    bool ok[3];
     for (int it = 0; it < 100; ++it) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -407,7 +431,7 @@ __device__ __forceinline__ void rattle_triangle(const double (&x)[3], const doub
                                       __dsub_rn(vz[b], vz[a]));
             ok[c] = !(fabs(rv) >= tol);
             if (fabs(rv) > tol) {
-                const double lam = rv / den[c];
+                const double lam = div_known(rv, tb.den[c], tb.rden[c]);
                 const double lx = __dmul_rn(lam, dx[c]), ly = __dmul_rn(lam, dy[c]), lz = __dmul_rn(lam, dz[c]);
                 vx[a] = __dadd_rn(vx[a], __dmul_rn(lx, w[a]));
                 vy[a] = __dadd_rn(vy[a], __dmul_rn(ly, w[a]));
@@ -432,31 +456,66 @@ __device__ __forceinline__ void rattle_triangle(const double (&x)[3], const doub
 // pending barostat scale), and SHAKE's displacement is also given to the
 // half-step velocities (v += dx / dt).
 __global__ void k_shake(Dev d) {
-    chain_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= d.n_cgroups) return;
-    const int r = d.cgroup_rep[g];
+    const bool in = g < d.n_cgroups;
+    // a triangle's data that the drift does not write are loaded before the wait
+    // for it (and the mirror's and the skin check's before the sweeps)
+    int r = 0, c0 = 0, c1 = 0;
+    int3 at;
+    bool tri = false;
+    int id[3], slot[3], im[3][3];
+    double w[3], dist[3], q[3], tc[3][3], xr[3][3];
+    if (in) {
+        r = d.cgroup_rep[g];
+        c0 = d.cgroup_begin[g];
+        c1 = d.cgroup_begin[g + 1];
+        tri = is_triangle(d, c0, c1, at);
+    }
+    if (tri) {
+        id[0] = at.x;
+        id[1] = at.y;
+        id[2] = at.z;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int a = id[k];
+            w[k] = 1.0 / d.mass[a];
+            dist[k] = d.cons_d[c0 + k];
+            q[k] = d.q[a];
+            slot[k] = d.slot_of_atom[a];
+            im[k][0] = d.imgx[a];
+            im[k][1] = d.imgy[a];
+            im[k][2] = d.imgz[a];
+            xr[k][0] = d.xr[a];
+            xr[k][1] = d.yr[a];
+            xr[k][2] = d.zr[a];
+            tc[k][0] = d.tcx[slot[k] >> 5];
+            tc[k][1] = d.tcy[slot[k] >> 5];
+            tc[k][2] = d.tcz[slot[k] >> 5];
+        }
+    }
+    chain_wait();
+    if (!in) return;
     RepState* s = d.st + r;
     if (!s->dr_move) return;  // the replicas k_kick_drift moved
     const Rep& R = d.rep[r];
     const bool phys = (R.flags & F_PHYS) != 0;
     const double L = phys ? s->dr_L * s->dr_pscale : s->dr_L, inv = 1.0 / L, tol = R.cons_tol;
-    const int c0 = d.cgroup_begin[g], c1 = d.cgroup_begin[g + 1];
-    const int q0 = d.cgroup_atom_begin[g], q1 = d.cgroup_atom_begin[g + 1];
     const int na = d.n_atoms;
-    int3 at;
-    if (is_triangle(d, c0, c1, at)) {
-        const int id[3] = {at.x, at.y, at.z};
-        double x[3], y[3], z[3], x0[3], y0[3], z0[3], w[3], dist[3];
+    if (tri) {
+        double x[3], y[3], z[3], x0[3], y0[3], z0[3], vx[3], vy[3], vz[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            x0[k] = x[k] = d.x[id[k]];
-            y0[k] = y[k] = d.y[id[k]];
-            z0[k] = z[k] = d.z[id[k]];
-            w[k] = 1.0 / d.mass[id[k]];
-            dist[k] = d.cons_d[c0 + k];
+            const int a = id[k];
+            x0[k] = x[k] = d.x[a];
+            y0[k] = y[k] = d.y[a];
+            z0[k] = z[k] = d.z[a];
+            vx[k] = d.vx[a];
+            vy[k] = d.vy[a];
+            vz[k] = d.vz[a];
         }
         shake_triangle(x, y, z, w, dist, L, inv, tol);
+        const double dt = R.dt, rdt = 1.0 / dt;
+        bool far = false;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const int a = id[k];
@@ -464,15 +523,24 @@ __global__ void k_shake(Dev d) {
             d.y[a] = y[k];
             d.z[a] = z[k];
             if (phys) {
-                d.vx[a] = __dadd_rn(d.vx[a], __dsub_rn(x[k], x0[k]) / R.dt);
-                d.vy[a] = __dadd_rn(d.vy[a], __dsub_rn(y[k], y0[k]) / R.dt);
-                d.vz[a] = __dadd_rn(d.vz[a], __dsub_rn(z[k], z0[k]) / R.dt);
+                d.vx[a] = __dadd_rn(vx[k], div_known(__dsub_rn(x[k], x0[k]), dt, rdt));
+                d.vy[a] = __dadd_rn(vy[k], div_known(__dsub_rn(y[k], y0[k]), dt, rdt));
+                d.vz[a] = __dadd_rn(vz[k], div_known(__dsub_rn(z[k], z0[k]), dt, rdt));
             }
-            write_mirror(d, d.slot_of_atom[a], a, x[k], y[k], z[k], L);
-            skin_check(d, s, R, a, x[k], y[k], z[k]);
+            // write_mirror and skin_check on the loaded values
+            if (d.xq32)
+                d.xq32[slot[k]] = make_float4(static_cast<float>((x[k] - im[k][0] * L) - tc[k][0]),
+                                              static_cast<float>((y[k] - im[k][1] * L) - tc[k][1]),
+                                              static_cast<float>((z[k] - im[k][2] * L) - tc[k][2]),
+                                              static_cast<float>(q[k]));
+            if (d.xq64) d.xq64[slot[k]] = make_double4(x[k], y[k], z[k], q[k]);
+            const double dx = x[k] - xr[k][0], dy = y[k] - xr[k][1], dz = z[k] - xr[k][2];
+            far |= dx * dx + dy * dy + dz * dz > R.half_skin2;
         }
+        if (phys && far) s->rebuild = 1;
         return;
     }
+    const int q0 = d.cgroup_atom_begin[g], q1 = d.cgroup_atom_begin[g + 1];
     if (phys)
         for (int q = q0; q < q1; ++q) {
             const int a = d.cgroup_atoms[q];
@@ -521,30 +589,48 @@ __global__ void k_shake(Dev d) {
 // Constraints::apply_rattle (constraints.cpp:49-91), after the second half
 // kick: the same group sweeps on r.v, lambda = r.v / (r^2 (1/m_i + 1/m_j)).
 __global__ void k_rattle(Dev d) {
-    chain_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= d.n_cgroups) return;
-    const int r = d.cgroup_rep[g];
-    RepState* s = d.st + r;
-    if (!s->active) return;
-    const Rep& R = d.rep[r];
-    const double L = s->L, inv = 1.0 / L, tol = R.cons_tol;
-    const int c0 = d.cgroup_begin[g], c1 = d.cgroup_begin[g + 1];
+    const bool in = g < d.n_cgroups;
+    // only the velocities come from the kernel before it
+    int r = 0, c0 = 0, c1 = 0;
     int3 at;
-    if (is_triangle(d, c0, c1, at)) {
-        const int id[3] = {at.x, at.y, at.z};
-        double x[3], y[3], z[3], vx[3], vy[3], vz[3], w[3];
+    bool tri = false, active = false;
+    double L = 1.0, inv = 1.0, tol = 0.0;
+    TriangleBonds tb;
+    double w[3];
+    if (in) {
+        r = d.cgroup_rep[g];
+        active = d.st[r].active != 0;
+        L = d.st[r].L;
+        inv = 1.0 / L;
+        tol = d.rep[r].cons_tol;
+        c0 = d.cgroup_begin[g];
+        c1 = d.cgroup_begin[g + 1];
+        tri = is_triangle(d, c0, c1, at);
+    }
+    const int id[3] = {at.x, at.y, at.z};
+    if (tri) {
+        double x[3], y[3], z[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             x[k] = d.x[id[k]];
             y[k] = d.y[id[k]];
             z[k] = d.z[id[k]];
+            w[k] = 1.0 / d.mass[id[k]];
+        }
+        tb.set(x, y, z, w, L, inv);
+    }
+    chain_wait();
+    if (!in || !active) return;
+    if (tri) {
+        double vx[3], vy[3], vz[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
             vx[k] = d.vx[id[k]];
             vy[k] = d.vy[id[k]];
             vz[k] = d.vz[id[k]];
-            w[k] = 1.0 / d.mass[id[k]];
         }
-        rattle_triangle(x, y, z, vx, vy, vz, w, L, inv, tol);
+        rattle_triangle(tb, vx, vy, vz, w, tol);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             d.vx[id[k]] = vx[k];
