@@ -1439,7 +1439,7 @@ void Batch::enqueue_eval(int pass) {
 
 // Neighbour-list rebuild: one cooperative launch that returns at once unless
 // some replica's rebuild flag is set.
-void Batch::enqueue_rebuild() { launch_rebuild(dev_, d_bin_rep_, n_sm_, stream_, &launches_); }
+void Batch::enqueue_rebuild() { launch_rebuild(dev_, d_bin_rep_, n_sm_, !any_pme_, stream_, &launches_); }
 
 // first: issue the first evaluation.  begun: the step before it in the same
 // launch began this one; next (NextStep): another step follows in the same
@@ -1807,7 +1807,7 @@ int Batch::rebuild_in_frame(const std::vector<char>& sel) {
     frame.x = dev_.xr;
     frame.y = dev_.yr;
     frame.z = dev_.zr;
-    launch_rebuild(frame, d_bin_rep_, n_sm_, stream_, &launches_);
+    launch_rebuild(frame, d_bin_rep_, n_sm_, false, stream_, &launches_);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream_));
     CK(cudaMemcpy(tmp.data(), d_st_, sizeof(RepState) * R, cudaMemcpyDeviceToHost));

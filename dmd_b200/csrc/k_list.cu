@@ -1513,7 +1513,8 @@ __device__ bool grid_barrier(const Dev& d) {
 // same flags, so a step without a rebuild leaves at once), then R1..R7 with a
 // grid barrier between phases.  Only replicas whose `rebuild` flag is set are
 // touched.
-__global__ void __launch_bounds__(NT_B, 4) k_rebuild(Dev d, const int* bin_rep) {
+__global__ void __launch_bounds__(NT_B, 4) k_rebuild(Dev d, const int* bin_rep, int chained) {
+    if (chained) chain_wait();
     int any = 0;
     for (int r = 0; r < d.n_rep; ++r) any |= d.st[r].rebuild;
     if (!any) return;
@@ -1661,7 +1662,7 @@ __global__ void __launch_bounds__(NT_B, 4) k_rebuild(Dev d, const int* bin_rep) 
         if (d.st[r].rebuild) d.st[r].rebuild = 0;
 }
 
-void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, cudaStream_t st, long long* nlaunch) {
+void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, bool chained, cudaStream_t st, long long* nlaunch) {
     static int per_sm = 0;  // co-resident blocks per SM (same on every device of one kind)
     if (per_sm == 0) {
         int n = 0;
@@ -1678,12 +1679,14 @@ void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, cudaStream_t st,
     cfg.blockDim = dim3(NT_B);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_rebuild, d, bin_rep);
+    cfg.numAttrs = chained ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, k_rebuild, d, bin_rep, chained ? 1 : 0);
     *nlaunch += 1;
 }
 

@@ -28,7 +28,11 @@ inline void launch_chained(void (*kernel)(P...), int grid, int block, cudaStream
 
 // k_list.cu: spatial sort + pair-list build for replicas whose `rebuild` flag
 // is set, as one cooperative launch (returns at once when no replica rebuilds).
-void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, cudaStream_t st, long long* nlaunch);
+// chained: launched as launch_chained does.  Only in tables without a PME chain:
+// 1,000 LJ atoms 1,721 -> 1,618 us per 100 steps, decane 4k 2,189 -> 2,095; with
+// one, the pair kernel's blocks then come before the chain's first ones and
+// water 9k went from 3,106 to 3,156 us per 50 steps.
+void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, bool chained, cudaStream_t st, long long* nlaunch);
 
 // k_nonbonded.cu: LJ + real-space Ewald over the pair list (replicas with `eval`).
 // Pair energies and virial are summed only for replicas whose `want_e` is set.

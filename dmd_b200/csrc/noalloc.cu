@@ -335,7 +335,7 @@ extern "C" int dmdgpu_nonbonded_noalloc(const dmdgpu_nb_params* p, const double*
     if (cudaGetLastError() != cudaSuccess) return DMDGPU_ERR_GPU;
     int n_sm = 148;
     if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return DMDGPU_ERR_GPU;
-    launch_rebuild(d, bin_rep, n_sm, st, &nl);
+    launch_rebuild(d, bin_rep, n_sm, false, st, &nl);
     if (cudaGetLastError() != cudaSuccess) return DMDGPU_ERR_GPU;
     launch_nonbonded(d, fp64, phys, n_sm, 2, NB_CHUNK32, st, &nl);
     if (cudaGetLastError() != cudaSuccess) return DMDGPU_ERR_GPU;
