@@ -809,7 +809,9 @@ int Batch::pack() {
             P.bsp_off = static_cast<int>(n_bsp);
             n_bsp += K;
             P.pme_block_begin = pme_blocks;
-            P.pme_blocks = static_cast<int>((static_cast<long long>(K) * K * (K / 2 + 1) + 256 * PME_POINTS - 1) / (256 * PME_POINTS));
+            const long long nc = static_cast<long long>(K) * K * (K / 2 + 1);
+            P.pme_points = nc >= 80000 ? PME_POINTS : 1;
+            P.pme_blocks = static_cast<int>((nc + 256 * P.pme_points - 1) / (256 * P.pme_points));
             pme_blocks += P.pme_blocks;
             P.conv_block_begin = conv_blocks;
             P.conv_points = P.mesh_fix_n >= (1 << 20) ? 4096 : 1024;

@@ -336,23 +336,19 @@ __device__ __forceinline__ bool mesh_coord(double x, double invL, int K, int& m0
     return ok;
 }
 
-// An atom's mesh coordinates and B-spline weights, formed once by G cooperating
-// lanes (a power of two >= 4, aligned; sub = lane within the group): lane k < 3
-// the coordinate of axis k, lane m the weights of stencil offset m & 3.  Every
-// lane of the group calls it.
+// An atom's mesh coordinates, formed once by G cooperating lanes (a power of two
+// >= 4, aligned): lane k < 3 of the group passes the atom's coordinate along axis
+// k.  Every lane of the group calls it.
 struct MeshPos {
     int m0[3];
     bool finite;
 };
 template <int G>
-__device__ __forceinline__ void mesh_position(const Dev& d, int a, double invL, int K, int sub, MeshPos& p,
-                                              double (&u)[3]) {
-    const int ax = sub < 3 ? sub : 0;
-    const double* xa = ax == 0 ? d.x : (ax == 1 ? d.y : d.z);
+__device__ __forceinline__ void mesh_position(double x, double invL, int K, MeshPos& p, double (&u)[3]) {
     int m;
     double v;
-    const bool ok = mesh_coord(xa[a], invL, K, m, v);
-    const unsigned grp = (G == 32 ? FULL : ((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1)));
+    const bool ok = mesh_coord(x, invL, K, m, v);
+    const unsigned grp = ((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
     p.finite = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -369,7 +365,7 @@ __device__ __forceinline__ void mesh_position(const Dev& d, int a, double invL, 
 // the fixed-point mesh on its own; the integer sums do not depend on order.
 // Bound by the L2's atomics (64 per atom) once the 16 lanes share the FP64
 // coordinates and the 12 weights instead of forming them 16 times: water 750k
-// 177 -> 156 us (308 G atomics/s).  Visiting the atoms in slot order with the
+// 177 -> 143 us (336 G atomics/s).  Visiting the atoms in slot order with the
 // next ones' data loaded ahead: 181 us.
 template <typename T>
 __global__ void k_pme_spread(Dev d) {
@@ -378,18 +374,20 @@ __global__ void k_pme_spread(Dev d) {
     const int a = static_cast<int>(t >> 4);
     // every condition below is uniform over the atom's 16 lanes
     if (a >= d.n_atoms) return;
+    const int sub = threadIdx.x & 15, ix = sub & 3, iy = sub >> 2;
+    // (independent loads first)
     const int r = d.atom_rep[a];
+    const double q = d.q[a];
+    const double xa = (sub == 1 ? d.y : (sub == 2 ? d.z : d.x))[a];
     RepState* s = d.st + r;
     const Rep& R = d.rep[r];
     if (!s->eval || !(R.flags & F_PME)) return;
-    const double q = d.q[a];
     if (q == 0.0) return;
     const int K = R.pme_K;
-    const int sub = threadIdx.x & 15, ix = sub & 3, iy = sub >> 2;
     const unsigned grp = 0xFFFFu << (threadIdx.x & 16);
     MeshPos p;
     double u[3];
-    mesh_position<16>(d, a, s->invL, K, sub, p, u);
+    mesh_position<16>(xa, s->invL, K, p, u);
     if (!p.finite && sub == 0) set_status(s, ST_NAN);
     // lane (axis, offset) = (iy, ix) for axis < 3 forms that weight
     const double ua = iy == 0 ? u[0] : (iy == 1 ? u[1] : u[2]);
@@ -428,7 +426,6 @@ __global__ void k_pme_spread(Dev d) {
 // harmless and no per-replica test delays the loads.
 template <typename T>
 __global__ void k_pme_convert(Dev d) {
-    chain_wait();
     const int r = d.conv_block_rep[blockIdx.x];
     const Rep& R = d.rep[r];
     const int ng = R.conv_points >> 10;  // groups per thread (1 or 4)
@@ -437,6 +434,7 @@ __global__ void k_pme_convert(Dev d) {
     long long* fix = d.mesh_fix + R.mesh_fix_off;
     T* real = reinterpret_cast<T*>(d.mesh_real) + R.mesh_real_off;
     const bool phys = (R.flags & F_PHYS) != 0;
+    chain_wait();  // the parameters above are the table's: loaded before the mesh is complete
     longlong2 v[8];
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -486,17 +484,15 @@ __global__ void k_pme_convert(Dev d) {
 // The influence function G depends only on the box, alpha and K: it is cached
 // (rounded to T) and recomputed only when the box edge changed (barostat, state
 // load).  Energy and virial sums are formed only when this evaluation's
-// energies are read.  PME_POINTS mesh points per thread, so that the FP64
-// reciprocals of the box terms, the block's sums and the partials k_replica_update
-// reads are shared by more points; under a barostat (G, energy and virial every
-// step) it is bound by the FP64 pipe: water 750k 69 -> 36 us.
-template <typename T>
-__global__ void k_pme_influence(Dev d) {
-    chain_wait();
-    const int r = d.pme_block_rep[blockIdx.x];
-    const Rep& R = d.rep[r];
-    RepState* s = d.st + r;
-    if (!s->eval) return;  // uniform over the block
+// energies are read.  Large meshes take PME_POINTS points per thread
+// (R.pme_points), so that the FP64 reciprocals of the box terms, the block's
+// sums and the partials k_replica_update reads are shared by more points (under a
+// barostat, G, energy and virial every step, the kernel is bound by the FP64
+// pipe: water 750k 69 -> 36 us, and beside the pair kernel fewer blocks wait for
+// a place: water 30k 9.2 against 5.5 us); small ones one, for enough blocks
+// (water 9k, 43^3: 3.6 -> 2.4 us).
+template <typename T, int NP>
+__device__ __forceinline__ void influence_block(const Dev& d, const Rep& R, RepState* s) {
     const int lb = blockIdx.x - R.pme_block_begin;
     const int K = R.pme_K, H = K / 2 + 1;
     const int nc = K * K * H;
@@ -504,11 +500,11 @@ __global__ void k_pme_influence(Dev d) {
     using C2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
     C2* cm = reinterpret_cast<C2*>(d.mesh_cplx) + R.mesh_cplx_off;
     T* gc = reinterpret_cast<T*>(d.pme_green) + R.mesh_cplx_off;
-    const int e0 = lb * (PME_POINTS * static_cast<int>(blockDim.x)) + static_cast<int>(threadIdx.x);
-    C2 z[PME_POINTS];
-    T green[PME_POINTS];
+    const int e0 = lb * (NP * static_cast<int>(blockDim.x)) + static_cast<int>(threadIdx.x);
+    C2 z[NP];
+    T green[NP];
 #pragma unroll
-    for (int q = 0; q < PME_POINTS; ++q) {
+    for (int q = 0; q < NP; ++q) {
         const int e = e0 + q * static_cast<int>(blockDim.x);
         z[q] = C2{0, 0};
         green[q] = 0;
@@ -528,7 +524,7 @@ __global__ void k_pme_influence(Dev d) {
         va = 1.0 / (2.0 * R.alpha * R.alpha);
     }
 #pragma unroll
-    for (int q = 0; q < PME_POINTS; ++q) {
+    for (int q = 0; q < NP; ++q) {
         const int e = e0 + q * static_cast<int>(blockDim.x);
         if (e >= nc) break;
         if (e == 0) {  // (0, 0, 0)
@@ -577,6 +573,17 @@ __global__ void k_pme_influence(Dev d) {
     }
 }
 
+template <typename T>
+__global__ void k_pme_influence(Dev d) {
+    chain_wait();
+    const int r = d.pme_block_rep[blockIdx.x];
+    const Rep& R = d.rep[r];
+    RepState* s = d.st + r;
+    if (!s->eval) return;  // uniform over the block
+    if (R.pme_points == 1) influence_block<T, 1>(d, R, s);
+    else influence_block<T, PME_POINTS>(d, R, s);
+}
+
 // interpolate_forces (coulomb_pme.cpp:205-283).  REF reads the potential with
 // the unpadded index from FFTW's padded buffer (padding reads as zero) and
 // scales it by 1/N (:303-306); PHYS reads the natural layout, unscaled.
@@ -585,8 +592,8 @@ __global__ void k_pme_influence(Dev d) {
 // order.  The lanes load along x (lane m the m-th point of each of the four
 // slices' rows: a warp instruction touches 8 lines, not 32) and exchange the
 // 4x4 block, and share the FP64 coordinates and the weights.  It was bound by
-// L1 line lookups and by forming 18 weights per thread: water 750k 150 -> 107 us,
-// water 9k 6.8 -> 5.6 us.
+// L1 line lookups and by forming 18 weights per thread: water 750k 150 -> 101 us,
+// water 9k 6.8 -> 6.0 us.
 template <typename T>
 __global__ void k_pme_gather(Dev d) {
     chain_wait();
@@ -594,21 +601,23 @@ __global__ void k_pme_gather(Dev d) {
     const int a = static_cast<int>(t >> 2);
     // every condition below is uniform over the atom's 4 lanes
     if (a >= d.n_atoms) return;
+    const int iz = threadIdx.x & 3;
+    // (independent loads first)
     const int r = d.atom_rep[a];
+    const double q = d.q[a];
+    const double xa = (iz == 1 ? d.y : (iz == 2 ? d.z : d.x))[a];
     RepState* s = d.st + r;
     const Rep& R = d.rep[r];
     if (!s->eval || !(R.flags & F_PME)) return;
-    const double q = d.q[a];
     if (q == 0.0) return;
     const int K = R.pme_K;
     const bool phys = (R.flags & F_PHYS) != 0;
     const int P = 2 * (K / 2 + 1);
     const double norm = 1.0 / (static_cast<double>(K) * K * K);
-    const int iz = threadIdx.x & 3;
     const unsigned grp = 0xFu << (threadIdx.x & 28);
     MeshPos p;
     double u[3];
-    mesh_position<4>(d, a, s->invL, K, iz, p, u);
+    mesh_position<4>(xa, s->invL, K, p, u);
     // lane m forms the weights of offset m on every axis
     const T tx = (T)(u[0] - (p.m0[0] + iz)), ty = (T)(u[1] - (p.m0[1] + iz)), tz = (T)(u[2] - (p.m0[2] + iz));
     const T wxl = theta4<T>(tx), dwxl = dtheta4<T>(tx), wyl = theta4<T>(ty), dwyl = dtheta4<T>(ty);

@@ -28,7 +28,7 @@ constexpr double MSCALE = 1099511627776.0;     // 2^40 per e (PME mesh charge)
 constexpr double FMAX = 1.0e9;                 // |F| above this -> BondExplosion status
 
 constexpr int WIDE_TILES = 4096;  // replicas of at least this many tiles are reduced by 512 threads
-constexpr int PME_POINTS = 4;  // mesh points per thread of the influence kernel (256 threads per block)
+constexpr int PME_POINTS = 4;  // most mesh points per thread of the influence kernel (256 threads per block)
 constexpr int EWALD_N = 24;  // coefficients of the FP64 path's real-space Ewald polynomial
 
 enum RepFlags : int {
@@ -63,6 +63,7 @@ struct Rep {
     long long mesh_cplx_off;             // K*K*(K/2+1) complex
     int bsp_off;                         // K doubles: B-spline factor per mesh index
     int pme_block_begin, pme_blocks;     // influence-kernel blocks
+    int pme_points;                      // its mesh points per thread (1 or PME_POINTS)
     int conv_block_begin, conv_blocks;   // convert-kernel blocks
     int conv_points;                     // mesh points per convert block (1,024 or 4,096)
     double rc_lj, rc_c, rc_list;
