@@ -254,9 +254,8 @@ Batch::Batch(const dmdgpu_options& opt, long long budget) : opt_(opt), budget_(b
     // first wherever an SM has room (the main stream's own kernels are
     // ordered by dependencies); in the step graph every kernel node but the
     // pair kernel's gets the higher priority.
-    configure_nonbonded_kernels();
     int prio_lo = 0, prio_hi = 0;
-    if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess ||
+    if (!configure_nonbonded_kernels() || cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess ||
         cudaStreamCreateWithPriority(&stream_, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
         cudaStreamCreateWithPriority(&aux_stream_, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
         cudaStreamCreateWithPriority(&bond_stream_, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||

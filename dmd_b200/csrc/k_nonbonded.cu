@@ -684,12 +684,25 @@ __global__ void __launch_bounds__(256, 2) k_nb8_f32(Dev d) {
 }
 
 // ---- all-FP64 path ----------------------------------------------------------
-// Per-warp staging of one chunk's j entries.
+// Per-warp staging of one chunk: both sides by component (a pair's lane reads any
+// entry of either), and its pairs, ordered by j, then i: first their codes
+// (32 j + i), then their forces.  384 pairs (most chunks hold about 200), so
+// that two blocks of 8 warps fit an SM; a fuller chunk is worked off in parts.
+constexpr int PAIRS64 = 384;
+union PairWord {
+    int code;
+    double f;
+};
 struct ChunkStage64 {
-    double4 xq[32];
-    int tj[32];
+    double ix[32], iy[32], iz[32], iw[32];
+    double jx[32], jy[32], jz[32], jw[32];
+    PairWord pair[PAIRS64];            // code, then F_x on j
+    double fy[PAIRS64], fz[PAIRS64];
+    double cf[EWALD_N];  // the replica's Ewald polynomial
+    float4 jf[32];   // j in single precision, for the distance test
+    uint2 row[32];   // of entry j: where its pairs begin, and their i as bits
+    int ti[32], tj[32];
     int js[32];
-    uint32_t mk[32];
 };
 
 // One chunk of a replica whose Ewald polynomial does not apply (alpha rc beyond
@@ -712,9 +725,12 @@ __device__ __noinline__ void nb_chunk_f64_erfc(const Dev& d, const Rep& R, RepSt
         xj = d.xq64[js];
         tj = d.type_s[js];
     }
-    S.xq[lane] = xj;
+    S.jx[lane] = xj.x;
+    S.jy[lane] = xj.y;
+    S.jz[lane] = xj.z;
+    S.jw[lane] = xj.w;
     S.tj[lane] = tj;
-    S.mk[lane] = mk;
+    S.js[lane] = static_cast<int>(mk);
     __syncwarp();
     const bool has_lj = (R.flags & F_LJ) != 0;
     const bool has_c = (R.flags & F_COUL_REAL) != 0;
@@ -724,9 +740,9 @@ __device__ __noinline__ void nb_chunk_f64_erfc(const Dev& d, const Rep& R, RepSt
     double el = 0, ec = 0, vir = 0;
     for (int k = 0; k < 32; ++k) {
         const int src = (lane + k) & 31;
-        const uint32_t m = S.mk[src];
+        const uint32_t m = static_cast<uint32_t>(S.js[src]);
         if ((m >> lane) & 1u) {
-            const double4 pj = S.xq[src];
+            const double4 pj = make_double4(S.jx[src], S.jy[src], S.jz[src], S.jw[src]);
             const double dx = mi_ref(__dsub_rn(pj.x, xi.x), L, invL);
             const double dy = mi_ref(__dsub_rn(pj.y, xi.y), L, invL);
             const double dz = mi_ref(__dsub_rn(pj.z, xi.z), L, invL);
@@ -785,19 +801,29 @@ __device__ __forceinline__ double rsqrt_h(double x) {
     return fma(y * h, fma(h, 0.375, 0.5), y);
 }
 
-// One chunk.  Bound by the FP64 pipe, so by what a pair costs in
-// it: a list entry's periodic image is the one frozen at the build (MI: the
-// box is narrower than twice the list cutoff, nearest image per pair), LJ and
-// the Ewald term share one reciprocal square root, and the Ewald term
+// One chunk.  About one lane pair in five lies inside a cutoff, and a round over
+// the tile's lanes costs its FP64 latency whether one lane or all take part.  So
+// the pairs are found first (single precision, against a bound no pair inside
+// exceeds), listed, and spread evenly over the lanes; their forces go to shared
+// memory, from which each lane sums those on its own entry and atom in the
+// list's order.  Water 30k, 22,800 chunks: 178 -> 145 us per launch, 24 % of
+// the FP64 pipe's cycles and 55 % of shared memory's; three blocks per SM (80
+// registers, spills) 161 us, the coefficients in registers (spills) 164 us,
+// a pair's force over r instead of its components 153 us.  4,000 argon atoms,
+// whose pair costs little, 2,123 -> 2,130 us per 60 steps, 16,384 3,428 -> 3,185.
+// What a pair costs: a list entry's periodic image is the one frozen at the
+// build (MI: the box is narrower than twice the list cutoff, nearest image per
+// pair), LJ and the Ewald term share one reciprocal square root, and the Ewald
+// term
 //   erfc(a r) / r^3 + 2 a / sqrt(pi) exp(-a^2 r^2) / r^2 = r^-3 - P(r^2)
 // with P(r^2) = erf(a r) / r^3 - 2 a / sqrt(pi) exp(-a^2 r^2) / r^2, which is
 // smooth in r^2 down to 0, as a polynomial fitted for the replica (EWALD_N
-// coefficients in registers) -- instead of a root, five divisions, erfc() and
-// exp().  Membership is the reference's: a pair within 1e-12 (relative) of a
-// cutoff is decided by its expression.  Energies (ENERGY) are formed beside the
-// same force arithmetic, with erfc(), so a force does not depend on whether its
-// evaluation's energies are read.  Water 30k, 22,800 chunks: 560 -> 177
-// us per launch.
+// coefficients in shared memory) -- instead of a root, five divisions, erfc()
+// and exp() (560 -> 177 us when that replaced them).  Membership is the
+// reference's: a pair within 1e-12 (relative) of a cutoff is decided by its
+// expression.  Energies (ENERGY) are formed beside the same force arithmetic,
+// with erfc(), so a force does not depend on whether its evaluation's energies
+// are read.
 template <bool COUL, bool MI, bool ENERGY>
 __device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
                                              ChunkStage64& S, Acc& acc) {
@@ -830,80 +856,153 @@ __device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepStat
             xj.z -= (d.imgz[aj] - (static_cast<int>((e >> 30) & 3u) - 1)) * L;
         }
     }
-    S.xq[lane] = xj;
+    S.ix[lane] = xi.x;
+    S.iy[lane] = xi.y;
+    S.iz[lane] = xi.z;
+    S.iw[lane] = KE * xi.w;
+    S.ti[lane] = ti;
+    S.jx[lane] = xj.x;
+    S.jy[lane] = xj.y;
+    S.jz[lane] = xj.z;
+    S.jw[lane] = xj.w;
     S.tj[lane] = tj;
     S.js[lane] = js;
-    uint32_t rm = rotated_columns(mk, lane);
+    if (!MI)
+        S.jf[lane] = make_float4(static_cast<float>(xj.x), static_cast<float>(xj.y), static_cast<float>(xj.z), 0.f);
+    if (COUL && lane < EWALD_N) S.cf[lane] = d.ewald_poly[EWALD_N * r + lane];
+    const uint32_t rot = rotated_columns(mk, lane);
+    const uint32_t col = __funnelshift_l(rot, rot, lane);  // bit j: (lane, entry j) interacts
     __syncwarp();
     const bool has_lj = (R.flags & F_LJ) != 0;
     const double rl2 = has_lj ? R.rc_lj2 : 0.0, rcc2 = COUL ? R.rc_c2 : 0.0;
     const double rmax2 = fmax(rl2, rcc2) * (1.0 + 1e-12);
     const double wl = rl2 * 1e-12, wc = rcc2 * 1e-12;
-    const double keqi = KE * xi.w;
-    double cf[EWALD_N];
-    double us = 0.0;
-    if (COUL) {
-        us = 2.0 / R.rc_c2;
-#pragma unroll
-        for (int k = 0; k < EWALD_N; ++k) cf[k] = d.ewald_poly[EWALD_N * r + k];
+
+    // The pairs that may lie inside a cutoff, entry by entry: every lane tests
+    // the same j, so the vote is j's row.  In single precision against a bound
+    // that no pair inside can exceed: with u = 2^-24, a component of the
+    // difference is off by at most 2 u (|x_i| + rmax) = err, r^2 by 2 sqrt(3)
+    // rmax err + 3 err^2 and 4 u of itself.
+    float thr = 0.f;
+    const float xf = static_cast<float>(xi.x), yf = static_cast<float>(xi.y), zf = static_cast<float>(xi.z);
+    if (!MI) {
+        const double rmax = sqrt(rmax2);
+        const double err = 1.2e-7 * (fmax(fmax(fabs(xi.x), fabs(xi.y)), fabs(xi.z)) + rmax);
+        thr = static_cast<float>(rmax2 * (1.0 + 1e-6) + 4.0 * (rmax + err) * err);
     }
-    const double2* lj = d.lj64 + R.lj_off + ti * R.n_types;
-    double fix = 0, fiy = 0, fiz = 0, fjx = 0, fjy = 0, fjz = 0;
-    double el = 0, ec = 0, vir = 0;
-    const int src_lane = (lane + 1) & 31;
-#pragma unroll 1
+    uint32_t nm = 0;
+#pragma unroll 8
     for (int k = 0; k < 32; ++k) {
-        const int src = (lane + k) & 31;
-        const double4 pj = S.xq[src];
-        double dx = pj.x - xi.x, dy = pj.y - xi.y, dz = pj.z - xi.z;
+        bool near;
         if (MI) {
+            double dx = S.jx[k] - xi.x, dy = S.jy[k] - xi.y, dz = S.jz[k] - xi.z;
             dx = fma(-L, rint(dx * invL), dx);
             dy = fma(-L, rint(dy * invL), dy);
             dz = fma(-L, rint(dz * invL), dz);
+            near = fma(dz, dz, fma(dy, dy, dx * dx)) < rmax2;
+        } else {
+            const float4 pj = S.jf[k];
+            const float dx = pj.x - xf, dy = pj.y - yf, dz = pj.z - zf;
+            near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < thr;
         }
-        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-        if ((rm & 1u) && r2 < rmax2) {
+        nm |= near ? 1u << k : 0u;
+    }
+    nm &= col;
+    const uint32_t below = (1u << lane) - 1u;
+    const double us = COUL ? 2.0 / R.rc_c2 : 0.0;
+    const double2* lj = d.lj64 + R.lj_off;
+    double el = 0, ec = 0, vir = 0;
+    double fix = 0, fiy = 0, fiz = 0, fjx = 0, fjy = 0, fjz = 0;
+    // four entries at a time while the list has room for their 128
+    for (int k0 = 0; k0 < 32;) {
+        const int first = k0;
+        int n = 0;
+        for (; k0 < 32 && n <= PAIRS64 - 128; k0 += 4) {
+#pragma unroll
+            for (int k1 = 0; k1 < 4; ++k1) {
+                const int k = k0 + k1;
+                const uint32_t row = __ballot_sync(FULL, (nm >> k) & 1u);
+                if (lane == 0) S.row[k] = make_uint2(static_cast<uint32_t>(n), row);
+                if ((nm >> k) & 1u) S.pair[n + __popc(row & below)].code = 32 * k + lane;
+                n += __popc(row);
+            }
+        }
+        __syncwarp();
+
+        // Each lane takes every 32nd pair, whoever its atoms are.
+#pragma unroll 1
+        for (int p = lane; p < n; p += 32) {
+            const int code = S.pair[p].code;
+            const int i = code & 31, j = code >> 5;
+            double dx = S.jx[j] - S.ix[i], dy = S.jy[j] - S.iy[i], dz = S.jz[j] - S.iz[i];
+            if (MI) {
+                dx = fma(-L, rint(dx * invL), dx);
+                dy = fma(-L, rint(dy * invL), dy);
+                dz = fma(-L, rint(dz * invL), dz);
+            }
+            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
             bool in_l = r2 < rl2, in_c = COUL && r2 < rcc2;
             if (fabs(r2 - rl2) < wl || (COUL && fabs(r2 - rcc2) < wc)) {
-                const int aj = d.atom_of_slot[S.js[src]];
-                in_l = has_lj && exact_inside(d, ai, aj, L, invL, R.rc_lj2);
-                in_c = COUL && exact_inside(d, ai, aj, L, invL, R.rc_c2);
+                const int ap = d.atom_of_slot[32 * I + i], aq = d.atom_of_slot[S.js[j]];
+                in_l = has_lj && exact_inside(d, ap, aq, L, invL, R.rc_lj2);
+                in_c = COUL && exact_inside(d, ap, aq, L, invL, R.rc_c2);
             }
             const double rinv = rsqrt_h(r2);
             const double ir2 = rinv * rinv;
             double f = 0.0;
             if (in_l) {
-                const double2 p = lj[S.tj[src]];
-                const double sr6 = p.y * (ir2 * ir2 * ir2);
-                f = 24.0 * p.x * ir2 * fma(2.0 * sr6, sr6, -sr6);
-                if (ENERGY) el = fma(4.0 * p.x, fma(sr6, sr6, -sr6), el);
+                const double2 c6 = lj[S.ti[i] * R.n_types + S.tj[j]];
+                const double sr6 = c6.y * (ir2 * ir2 * ir2);
+                f = 24.0 * c6.x * ir2 * fma(2.0 * sr6, sr6, -sr6);
+                if (ENERGY) el = fma(4.0 * c6.x, fma(sr6, sr6, -sr6), el);
             }
             if (COUL) {
                 const double u = fma(r2, us, -1.0);
                 const double u2 = u * u;  // even and odd powers: two chains
-                double qe = cf[EWALD_N - 2], qo = cf[EWALD_N - 1];
+                double qe = S.cf[EWALD_N - 2], qo = S.cf[EWALD_N - 1];
 #pragma unroll
-                for (int n = EWALD_N - 4; n >= 0; n -= 2) {
-                    qe = fma(qe, u2, cf[n]);
-                    qo = fma(qo, u2, cf[n + 1]);
+                for (int m = EWALD_N - 4; m >= 0; m -= 2) {
+                    qe = fma(qe, u2, S.cf[m]);
+                    qo = fma(qo, u2, S.cf[m + 1]);
                 }
-                const double q = fma(qo, u, qe);
-                const double fc = keqi * pj.w * fma(rinv, ir2, -q);
+                const double qq = S.iw[i] * S.jw[j];
+                const double fc = qq * fma(rinv, ir2, -fma(qo, u, qe));
                 f += in_c ? fc : 0.0;
-                if (ENERGY && in_c) ec = fma(keqi * pj.w * rinv, erfc(R.alpha * (r2 * rinv)), ec);
+                if (ENERGY && in_c) ec = fma(qq * rinv, erfc(R.alpha * (r2 * rinv)), ec);
             }
             if (ENERGY) vir = fma(f, r2, vir);
-            fix = fma(-f, dx, fix);
-            fiy = fma(-f, dy, fiy);
-            fiz = fma(-f, dz, fiz);
-            fjx = fma(f, dx, fjx);
-            fjy = fma(f, dy, fjy);
-            fjz = fma(f, dz, fjz);
+            S.pair[p].f = f * dx;
+            S.fy[p] = f * dy;
+            S.fz[p] = f * dz;
         }
-        rm >>= 1;
-        fjx = __shfl_sync(FULL, fjx, src_lane);
-        fjy = __shfl_sync(FULL, fjy, src_lane);
-        fjz = __shfl_sync(FULL, fjz, src_lane);
+        __syncwarp();
+
+        // Lane l sums the forces on entry l, then on atom l of the tile.
+        const uint2 own = S.row[lane];
+        const uint32_t end = (lane >= first && lane < k0) ? own.x + __popc(own.y) : 0u;
+#pragma unroll 4
+        for (uint32_t p = own.x; p < end; ++p) {
+            fjx += S.pair[p].f;
+            fjy += S.fy[p];
+            fjz += S.fz[p];
+        }
+        uint32_t im = nm & (0xFFFFFFFFu >> (32 - k0)) & (0xFFFFFFFFu << first);
+        while (im) {  // two entries a turn, their loads side by side
+            const uint2 r0 = S.row[__ffs(im) - 1];
+            im &= im - 1u;
+            const bool two = im != 0;
+            const uint2 r1 = two ? S.row[__ffs(im) - 1] : r0;
+            im &= im - 1u;
+            const uint32_t p = r0.x + __popc(r0.y & below), q = r1.x + __popc(r1.y & below);
+            const double gx = S.pair[q].f, gy = S.fy[q], gz = S.fz[q];
+            fix -= S.pair[p].f;
+            fiy -= S.fy[p];
+            fiz -= S.fz[p];
+            fix -= two ? gx : 0.0;
+            fiy -= two ? gy : 0.0;
+            fiz -= two ? gz : 0.0;
+        }
+        __syncwarp();
     }
     if (ai >= 0) {
         fix_add(d.fnx + si, to_fix(fix, FSCALE, s));
@@ -931,14 +1030,13 @@ __device__ __noinline__ void nb_chunk_f64_energy(const Dev& d, const Rep& R, Rep
 }
 
 // Persistent, chunks claimed as in k_nb_f32 (first chunk without a claim).
-// PHYS tables with real-space Coulomb hold the Ewald coefficients in registers
-// (2 blocks of 256 threads per SM).
+// 2 blocks of 256 threads per SM, by registers and by shared memory.
 template <bool PHYS>
 __global__ void __launch_bounds__(256, 2) k_nb_f64(const __grid_constant__ Dev d) {
     chain_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    __shared__ ChunkStage64 s_stage[8];
+    extern __shared__ ChunkStage64 s_stage[];  // one per warp
     const int nw = gridDim.x * 8;
     const int total = d.chunk_prefix[d.n_rep];
     Acc acc{0, 0, 0};
@@ -988,6 +1086,7 @@ __global__ void __launch_bounds__(256, 2) k_nb_f64(const __grid_constant__ Dev d
 }  // namespace
 
 namespace {
+constexpr int NB64_SMEM = 8 * static_cast<int>(sizeof(ChunkStage64));
 const void* const kNbKernels[] = {
     reinterpret_cast<const void*>(k_nb_f32<true, true, false>),
     reinterpret_cast<const void*>(k_nb_f32<true, false, false>),
@@ -1017,18 +1116,26 @@ bool is_nonbonded_kernel(const void* f) {
 // kernels (4-16 KB of shared memory per block) cannot start beside it: on
 // water 30k they waited ~24 us for its last blocks.  A carveout of 60 % of the
 // unified L1 / shared memory as shared memory leaves room for them; the SPME
-// chain then runs during the pair kernel (step period 140 -> 128 us).
-void configure_nonbonded_kernels() {
+// chain then runs during the pair kernel (step period 140 -> 128 us).  The FP64
+// kernel fills the registers with two blocks per SM, so nothing runs beside it;
+// it takes the shared memory its two blocks need.
+bool configure_nonbonded_kernels() {
     for (const void* k : kNbKernels)
         if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 60) != cudaSuccess)
             cudaGetLastError();
+    for (const void* k : {reinterpret_cast<const void*>(k_nb_f64<true>), reinterpret_cast<const void*>(k_nb_f64<false>)}) {
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, NB64_SMEM) != cudaSuccess) return false;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
+            cudaGetLastError();
+    }
+    return true;
 }
 
 void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_per_sm, int form,
                       cudaStream_t st, long long* nlaunch) {
     if (fp64) {
-        if (phys) launch_chained(k_nb_f64<true>, n_sm * 2, 256, st, d);
-        else launch_chained(k_nb_f64<false>, n_sm * 2, 256, st, d);
+        if (phys) launch_chained_smem(k_nb_f64<true>, n_sm * 2, 256, NB64_SMEM, st, d);
+        else launch_chained_smem(k_nb_f64<false>, n_sm * 2, 256, NB64_SMEM, st, d);
     } else {
         const bool ljs = d.n_lj <= LJ_SMEM;
         // a table without real-space Coulomb runs the LJ-only instantiation

@@ -13,10 +13,11 @@ namespace dmd {
 // launched this way calls chain_wait() before it touches memory.  Saves about
 // 1 us of launch latency per kernel of the step's chain.
 template <typename... P, typename... A>
-inline void launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... args) {
+inline void launch_chained_smem(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));
     cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -24,6 +25,10 @@ inline void launch_chained(void (*kernel)(P...), int grid, int block, cudaStream
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... args) {
+    launch_chained_smem(kernel, grid, block, 0, st, args...);
 }
 
 // k_list.cu: spatial sort + pair-list build for replicas whose `rebuild` flag
@@ -37,10 +42,11 @@ void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, bool chained, cu
 // k_nonbonded.cu: LJ + real-space Ewald over the pair list (replicas with `eval`).
 // Pair energies and virial are summed only for replicas whose `want_e` is set.
 // The mixed-precision kernels are persistent with blocks_per_sm blocks of 256
-// threads per SM (1..3) and come in two forms -- one warp per 32 x 32 chunk,
-// or one warp per 8-atom i-cluster over its rows (needs d.cl_j) -- both chosen
-// by the engine's autotuner; results do not depend on the launch shape (one
-// warp per work item, fixed-point sums).
+// threads per SM (1..3, LJ only 1..4) and come in two forms -- one warp per
+// 32 x 32 chunk, or one warp per 8-atom i-cluster over its rows (needs d.cl_j).
+// The form is the caller's option; the blocks follow from the list's size, a
+// single system with a PME chain timing the other shapes too.  Results do not
+// depend on the launch shape (one warp per work item, fixed-point sums).
 enum NbForm { NB_CHUNK32 = 0, NB_CLUSTER8 = 1 };
 void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_per_sm, int form,
                       cudaStream_t st, long long* nlaunch);
@@ -48,8 +54,9 @@ void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_p
 // pair kernels: the step graph gives every other kernel the higher priority.
 bool is_nonbonded_kernel(const void* func);
 // Per-device function attributes of the pair kernels (the shared-memory
-// carveout); called once per context before the first launch.
-void configure_nonbonded_kernels();
+// carveout and limit); called once per context before the first launch.  False
+// where the device refuses the FP64 kernel's shared memory.
+bool configure_nonbonded_kernels();
 
 // k_forces.cu
 // bonds, angles, dihedrals and the exclusion correction in one launch

@@ -214,3 +214,22 @@ def test_ref_cadence_in_batch(oracle):
         assert b.scalars(k).step == n
         assert np.abs(b.positions(k) - oe.get(0)).max() < 1e-9
         assert rel_rms(b.velocities(k), oe.get(1)) < 1e-9
+
+
+@pytest.mark.parametrize("far", [0, 1000])
+@pytest.mark.parametrize("n,d", [(33, 0.34), (64, 0.34), (64, 0.2), (700, 0.3)])
+def test_fp64_dense_chunks(oracle, n, d, far):
+    """FP64 pair kernel on dense clusters (64 atoms 0.2 nm apart: every pair of a
+    chunk within the cutoff, its list full) and with atoms many boxes from the
+    origin, where the single-precision distance test must not drop a pair.
+    Tolerance: 1e-9 (the fixed-point step); 1,000 boxes out the coordinates hold
+    1e-12 nm, on forces that change 14-fold per distance: 1e-9 still."""
+    rng = np.random.default_rng(n)
+    m = math.ceil(n ** (1 / 3) - 1e-9)
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    w = W.lj_fluid(n, 0.1, 1.0, seed=3)
+    w.pos = (g + 0.02 * rng.random((n, 3))) * d + 0.1 + far * w.box * rng.integers(-1, 2, (n, 3))
+    c = w.config()
+    f, _ = _engine(c, "fp64", "phys").compute_forces()
+    f_o, _ = oracle.forces(c, "phys")
+    assert rel_rms(f, f_o) < 1e-9
