@@ -231,11 +231,11 @@ class Batch {
     bool failed_ = false;
     bool graph_dirty_ = true;
     bool need_eval1_ = true;
-    int nb_blocks_per_sm_ = 2;  // pair-kernel launch shape (autotuned)
+    int nb_blocks_per_sm_ = 2;  // pair-kernel launch shape (pack(), autotune())
     int prio_lo_ = 0, prio_hi_ = 0;  // stream priority range
     double density_ = 0.0;           // table atoms per nm^3 (autotuner cache key)
     void set_node_priorities(cudaGraph_t g);
-    int nb_form_ = 1;           // pair-kernel form (NbForm; autotuned)
+    int nb_form_ = 1;           // pair-kernel form (NbForm), from the options
     bool tuned_ = false;
     bool rule_bps_ = false;     // the launch shape follows from the table (no PME chain)
     std::vector<int> n_chunks_built_;  // chunks per packed replica at its last build in frame

@@ -9,8 +9,9 @@
 //   k_kick_drift        pending thermostat scale, half kick, PHYS pending
 //                       barostat scale, drift, clear forces, write the sorted
 //                       FP32/FP64 mirror, skin check (replicas with step < target)
-//   [eval #2]           (its k_eval_begin marks the replicas that advance and
-//                       scales the PHYS box to match the drift)
+//   [eval #2]           (k_eval_begin, launched before the drift or, between the
+//                       steps of one graph, done by k_replica_update, marks the
+//                       replicas that advance and scales the PHYS box to match)
 //   k_kick2             half kick (+ Andersen), per-tile KE / virial partials
 //   k_replica_update    closes eval #2, KE, thermostat (Berendsen / Nose-Hoover
 //                       scale, applied lazily in the next kick), Berendsen
