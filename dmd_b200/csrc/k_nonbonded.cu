@@ -806,11 +806,12 @@ __device__ __forceinline__ double rsqrt_h(double x) {
 // the pairs are found first (single precision, against a bound no pair inside
 // exceeds), listed, and spread evenly over the lanes; their forces go to shared
 // memory, from which each lane sums those on its own entry and atom in the
-// list's order.  Water 30k, 22,800 chunks: 178 -> 145 us per launch, 24 % of
-// the FP64 pipe's cycles and 55 % of shared memory's; three blocks per SM (80
+// list's order.  Water 30k, 22,800 chunks: 178 -> 139 us per launch, 25 % of
+// the FP64 pipe's cycles and 70 % of the L1 / shared data path's; three blocks per SM (80
 // registers, spills) 161 us, the coefficients in registers (spills) 164 us,
-// a pair's force over r instead of its components 153 us.  4,000 argon atoms,
-// whose pair costs little, 2,123 -> 2,130 us per 60 steps, 16,384 3,428 -> 3,185.
+// a pair's force over r instead of its components 153 us, one pair a turn instead
+// of two 145 us.  4,000 argon atoms, whose pair costs little, 2,123 -> 2,097 us
+// per 60 steps, 16,384 3,428 -> 3,207.
 // What a pair costs: a list entry's periodic image is the one frozen at the
 // build (MI: the box is narrower than twice the list cutoff, nearest image per
 // pair), LJ and the Ewald term share one reciprocal square root, and the Ewald
@@ -929,51 +930,86 @@ __device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepStat
         }
         __syncwarp();
 
-        // Each lane takes every 32nd pair, whoever its atoms are.
+        // Each lane takes every 32nd pair, whoever its atoms are, two at a time:
+        // their arithmetic side by side, one read of a coefficient for both.
 #pragma unroll 1
-        for (int p = lane; p < n; p += 32) {
-            const int code = S.pair[p].code;
-            const int i = code & 31, j = code >> 5;
-            double dx = S.jx[j] - S.ix[i], dy = S.jy[j] - S.iy[i], dz = S.jz[j] - S.iz[i];
-            if (MI) {
-                dx = fma(-L, rint(dx * invL), dx);
-                dy = fma(-L, rint(dy * invL), dy);
-                dz = fma(-L, rint(dz * invL), dz);
+        for (int p = lane; p < n; p += 64) {
+            const bool two = p + 32 < n;
+            const int code[2] = {S.pair[p].code, S.pair[two ? p + 32 : p].code};
+            double dx[2], dy[2], dz[2], r2[2], rinv[2], f[2], qe[2], qo[2], u[2], u2[2];
+            bool in_l[2], in_c[2], band = false;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = code[h] & 31, j = code[h] >> 5;
+                dx[h] = S.jx[j] - S.ix[i];
+                dy[h] = S.jy[j] - S.iy[i];
+                dz[h] = S.jz[j] - S.iz[i];
+                if (MI) {
+                    dx[h] = fma(-L, rint(dx[h] * invL), dx[h]);
+                    dy[h] = fma(-L, rint(dy[h] * invL), dy[h]);
+                    dz[h] = fma(-L, rint(dz[h] * invL), dz[h]);
+                }
+                r2[h] = fma(dz[h], dz[h], fma(dy[h], dy[h], dx[h] * dx[h]));
+                in_l[h] = r2[h] < rl2;
+                in_c[h] = COUL && r2[h] < rcc2;
+                band = band || fabs(r2[h] - rl2) < wl || (COUL && fabs(r2[h] - rcc2) < wc);
+                rinv[h] = rsqrt_h(r2[h]);
+                f[h] = 0.0;
             }
-            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-            bool in_l = r2 < rl2, in_c = COUL && r2 < rcc2;
-            if (fabs(r2 - rl2) < wl || (COUL && fabs(r2 - rcc2) < wc)) {
-                const int ap = d.atom_of_slot[32 * I + i], aq = d.atom_of_slot[S.js[j]];
-                in_l = has_lj && exact_inside(d, ap, aq, L, invL, R.rc_lj2);
-                in_c = COUL && exact_inside(d, ap, aq, L, invL, R.rc_c2);
+            if (band) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (fabs(r2[h] - rl2) < wl || (COUL && fabs(r2[h] - rcc2) < wc)) {
+                        const int ap = d.atom_of_slot[32 * I + (code[h] & 31)], aq = d.atom_of_slot[S.js[code[h] >> 5]];
+                        in_l[h] = has_lj && exact_inside(d, ap, aq, L, invL, R.rc_lj2);
+                        in_c[h] = COUL && exact_inside(d, ap, aq, L, invL, R.rc_c2);
+                    }
+                }
             }
-            const double rinv = rsqrt_h(r2);
-            const double ir2 = rinv * rinv;
-            double f = 0.0;
-            if (in_l) {
-                const double2 c6 = lj[S.ti[i] * R.n_types + S.tj[j]];
-                const double sr6 = c6.y * (ir2 * ir2 * ir2);
-                f = 24.0 * c6.x * ir2 * fma(2.0 * sr6, sr6, -sr6);
-                if (ENERGY) el = fma(4.0 * c6.x, fma(sr6, sr6, -sr6), el);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (in_l[h]) {
+                    const double ir2 = rinv[h] * rinv[h];
+                    const double2 c6 = lj[S.ti[code[h] & 31] * R.n_types + S.tj[code[h] >> 5]];
+                    const double sr6 = c6.y * (ir2 * ir2 * ir2);
+                    f[h] = 24.0 * c6.x * ir2 * fma(2.0 * sr6, sr6, -sr6);
+                    if (ENERGY && (h == 0 || two)) el = fma(4.0 * c6.x, fma(sr6, sr6, -sr6), el);
+                }
             }
             if (COUL) {
-                const double u = fma(r2, us, -1.0);
-                const double u2 = u * u;  // even and odd powers: two chains
-                double qe = S.cf[EWALD_N - 2], qo = S.cf[EWALD_N - 1];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    u[h] = fma(r2[h], us, -1.0);
+                    u2[h] = u[h] * u[h];  // even and odd powers: two chains
+                    qe[h] = S.cf[EWALD_N - 2];
+                    qo[h] = S.cf[EWALD_N - 1];
+                }
 #pragma unroll
                 for (int m = EWALD_N - 4; m >= 0; m -= 2) {
-                    qe = fma(qe, u2, S.cf[m]);
-                    qo = fma(qo, u2, S.cf[m + 1]);
+                    const double ce = S.cf[m], co = S.cf[m + 1];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        qe[h] = fma(qe[h], u2[h], ce);
+                        qo[h] = fma(qo[h], u2[h], co);
+                    }
                 }
-                const double qq = S.iw[i] * S.jw[j];
-                const double fc = qq * fma(rinv, ir2, -fma(qo, u, qe));
-                f += in_c ? fc : 0.0;
-                if (ENERGY && in_c) ec = fma(qq * rinv, erfc(R.alpha * (r2 * rinv)), ec);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double qq = S.iw[code[h] & 31] * S.jw[code[h] >> 5];
+                    const double fc = qq * fma(rinv[h], rinv[h] * rinv[h], -fma(qo[h], u[h], qe[h]));
+                    f[h] += in_c[h] ? fc : 0.0;
+                    if (ENERGY && in_c[h] && (h == 0 || two))
+                        ec = fma(qq * rinv[h], erfc(R.alpha * (r2[h] * rinv[h])), ec);
+                }
             }
-            if (ENERGY) vir = fma(f, r2, vir);
-            S.pair[p].f = f * dx;
-            S.fy[p] = f * dy;
-            S.fz[p] = f * dz;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (h == 1 && !two) continue;
+                if (ENERGY) vir = fma(f[h], r2[h], vir);
+                S.pair[p + 32 * h].f = f[h] * dx[h];
+                S.fy[p + 32 * h] = f[h] * dy[h];
+                S.fz[p + 32 * h] = f[h] * dz[h];
+            }
         }
         __syncwarp();
 
