@@ -814,7 +814,11 @@ __device__ __forceinline__ double rsqrt_h(double x) {
 // per 60 steps, 16,384 3,428 -> 3,207.
 // What a pair costs: a list entry's periodic image is the one frozen at the
 // build (MI: the box is narrower than twice the list cutoff, nearest image per
-// pair), LJ and the Ewald term share one reciprocal square root, and the Ewald
+// pair).  The PHYS list's skin sees to it that no pair inside a cutoff has left
+// that image.  The REF list has none and is kept for five steps, so there the
+// distance test also looks for pairs half a box apart or more (CHECK), the only
+// ones whose nearest image can be another: the chunk is then left undone (false)
+// and done over with MI (16,384 argon atoms 2,557 -> 2,584 us per 50 steps).  LJ and the Ewald term share one reciprocal square root, and the Ewald
 // term
 //   erfc(a r) / r^3 + 2 a / sqrt(pi) exp(-a^2 r^2) / r^2 = r^-3 - P(r^2)
 // with P(r^2) = erf(a r) / r^3 - 2 a / sqrt(pi) exp(-a^2 r^2) / r^2, which is
@@ -825,8 +829,8 @@ __device__ __forceinline__ double rsqrt_h(double x) {
 // expression.  Energies (ENERGY) are formed beside the same force arithmetic,
 // with erfc(), so a force does not depend on whether its evaluation's energies
 // are read.
-template <bool COUL, bool MI, bool ENERGY>
-__device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
+template <bool COUL, bool MI, bool ENERGY, bool CHECK>
+__device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
                                              ChunkStage64& S, Acc& acc) {
     const double L = s->L, invL = s->invL;
     const int I = d.chunk_itile[c];
@@ -884,14 +888,20 @@ __device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepStat
     // that no pair inside can exceed: with u = 2^-24, a component of the
     // difference is off by at most 2 u (|x_i| + rmax) = err, r^2 by 2 sqrt(3)
     // rmax err + 3 err^2 and 4 u of itself.
-    float thr = 0.f;
+    // The same for half a box (hl2), from below.
+    float thr = 0.f, hl2 = 0.f;
     const float xf = static_cast<float>(xi.x), yf = static_cast<float>(xi.y), zf = static_cast<float>(xi.z);
     if (!MI) {
         const double rmax = sqrt(rmax2);
-        const double err = 1.2e-7 * (fmax(fmax(fabs(xi.x), fabs(xi.y)), fabs(xi.z)) + rmax);
+        const double xmax = fmax(fmax(fabs(xi.x), fabs(xi.y)), fabs(xi.z));
+        const double err = 1.2e-7 * (xmax + rmax);
         thr = static_cast<float>(rmax2 * (1.0 + 1e-6) + 4.0 * (rmax + err) * err);
+        if (CHECK) {
+            const double h = 0.5 * L, herr = 1.2e-7 * (xmax + h);
+            hl2 = static_cast<float>(h * h * (1.0 - 1e-6) - 4.0 * (h + herr) * herr);
+        }
     }
-    uint32_t nm = 0;
+    uint32_t nm = 0, far = 0;
 #pragma unroll 8
     for (int k = 0; k < 32; ++k) {
         bool near;
@@ -904,9 +914,15 @@ __device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepStat
         } else {
             const float4 pj = S.jf[k];
             const float dx = pj.x - xf, dy = pj.y - yf, dz = pj.z - zf;
-            near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < thr;
+            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            near = r2 < thr;
+            if (CHECK) far |= r2 >= hl2 ? 1u << k : 0u;
         }
         nm |= near ? 1u << k : 0u;
+    }
+    if (CHECK && __any_sync(FULL, (far & col) != 0)) {
+        __syncwarp();  // the staged entries have been read
+        return false;
     }
     nm &= col;
     const uint32_t below = (1u << lane) - 1u;
@@ -1056,13 +1072,14 @@ __device__ __forceinline__ void nb_chunk_f64(const Dev& d, const Rep& R, RepStat
         acc.v += to_fix(vir, ESCALE, s);
     }
     __syncwarp();
+    return true;
 }
 
 // The energy forms, out of line: their registers do not weigh on the others.
-template <bool COUL, bool MI>
-__device__ __noinline__ void nb_chunk_f64_energy(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
+template <bool COUL, bool MI, bool CHECK>
+__device__ __noinline__ bool nb_chunk_f64_energy(const Dev& d, const Rep& R, RepState* s, int r, int c, int lane,
                                                  ChunkStage64& S, Acc& acc) {
-    nb_chunk_f64<COUL, MI, true>(d, R, s, r, c, lane, S, acc);
+    return nb_chunk_f64<COUL, MI, true, CHECK>(d, R, s, r, c, lane, S, acc);
 }
 
 // Persistent, chunks claimed as in k_nb_f32 (first chunk without a claim).
@@ -1089,22 +1106,20 @@ __global__ void __launch_bounds__(256, 2) k_nb_f64(const __grid_constant__ Dev d
         if (s->eval) {
             const int c = R.chunk_begin + (w - d.chunk_prefix[r]);
             const bool coul = PHYS && (R.flags & F_COUL_REAL);
-            const bool mi = 4.0 * R.rc_list2 > s->L * s->L;
+            bool mi = 4.0 * R.rc_list2 > s->L * s->L;
+            ChunkStage64& S = s_stage[wib];
             if (coul && !R.ewald_ok) {
-                nb_chunk_f64_erfc(d, R, s, c, lane, s_stage[wib], acc);
+                nb_chunk_f64_erfc(d, R, s, c, lane, S, acc);
             } else if (s->want_e) {
-                if (coul && !mi) nb_chunk_f64_energy<PHYS, false>(d, R, s, r, c, lane, s_stage[wib], acc);
-                else if (coul) nb_chunk_f64_energy<PHYS, true>(d, R, s, r, c, lane, s_stage[wib], acc);
-                else if (!mi) nb_chunk_f64_energy<false, false>(d, R, s, r, c, lane, s_stage[wib], acc);
-                else nb_chunk_f64_energy<false, true>(d, R, s, r, c, lane, s_stage[wib], acc);
-            } else if (coul && !mi) {
-                nb_chunk_f64<PHYS, false, false>(d, R, s, r, c, lane, s_stage[wib], acc);
-            } else if (coul) {
-                nb_chunk_f64<PHYS, true, false>(d, R, s, r, c, lane, s_stage[wib], acc);
-            } else if (!mi) {
-                nb_chunk_f64<false, false, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+                if (coul && !mi) nb_chunk_f64_energy<PHYS, false, false>(d, R, s, r, c, lane, S, acc);
+                else if (!mi) mi = !nb_chunk_f64_energy<false, false, !PHYS>(d, R, s, r, c, lane, S, acc);
+                if (coul && mi) nb_chunk_f64_energy<PHYS, true, false>(d, R, s, r, c, lane, S, acc);
+                else if (mi) nb_chunk_f64_energy<false, true, false>(d, R, s, r, c, lane, S, acc);
             } else {
-                nb_chunk_f64<false, true, false>(d, R, s, r, c, lane, s_stage[wib], acc);
+                if (coul && !mi) nb_chunk_f64<PHYS, false, false, false>(d, R, s, r, c, lane, S, acc);
+                else if (!mi) mi = !nb_chunk_f64<false, false, false, !PHYS>(d, R, s, r, c, lane, S, acc);
+                if (coul && mi) nb_chunk_f64<PHYS, true, false, false>(d, R, s, r, c, lane, S, acc);
+                else if (mi) nb_chunk_f64<false, true, false, false>(d, R, s, r, c, lane, S, acc);
             }
         } else {
             skip = d.chunk_prefix[r + 1] - nw;  // past this replica's chunks

@@ -233,3 +233,21 @@ def test_fp64_dense_chunks(oracle, n, d, far):
     f, _ = _engine(c, "fp64", "phys").compute_forces()
     f_o, _ = oracle.forces(c, "phys")
     assert rel_rms(f, f_o) < 1e-9
+
+
+@pytest.mark.parametrize("half", [0.5, 0.4995])
+def test_fp64_ref_box_of_two_cutoffs(oracle, half):
+    """REF keeps a list without a skin for five steps.  In a box of two cutoffs (or
+    just above) the nearest image of a listed pair changes in between (up to 17
+    pairs at a time here), and FP64 forces follow it as the oracle's do, over four
+    cadences.  Tolerances: 1e-8 for a force component (at most 64 contributions
+    to an atom of 8 tiles, each rounded to 2^-32; a pair lost at the cutoff is
+    worth 1e-2) and 1e-9 nm."""
+    c = _argon(4, 1)
+    c.lj_cutoff = half * c.box_size
+    oe, eng = oracle.engine(c, "ref"), _engine(c, "fp64", "ref")
+    for _ in range(21):
+        oe.step(1)
+        eng.run_n(1)
+        assert np.abs(eng.forces - oe.get(2)).max() < 1e-8
+        assert np.abs(eng.positions - oe.get(0)).max() < 1e-9
