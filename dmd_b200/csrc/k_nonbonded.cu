@@ -960,10 +960,10 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
                 dx[h] = S.jx[j] - S.ix[i];
                 dy[h] = S.jy[j] - S.iy[i];
                 dz[h] = S.jz[j] - S.iz[i];
-                if (MI) {
-                    dx[h] = fma(-L, rint(dx[h] * invL), dx[h]);
-                    dy[h] = fma(-L, rint(dy[h] * invL), dy[h]);
-                    dz[h] = fma(-L, rint(dz[h] * invL), dz[h]);
+                if (MI) {  // (exactly half a box apart: away from zero, as the reference rounds)
+                    dx[h] = fma(-L, round(dx[h] * invL), dx[h]);
+                    dy[h] = fma(-L, round(dy[h] * invL), dy[h]);
+                    dz[h] = fma(-L, round(dz[h] * invL), dz[h]);
                 }
                 r2[h] = fma(dz[h], dz[h], fma(dy[h], dy[h], dx[h] * dx[h]));
                 in_l[h] = r2[h] < rl2;

@@ -251,3 +251,19 @@ def test_fp64_ref_box_of_two_cutoffs(oracle, half):
         eng.run_n(1)
         assert np.abs(eng.forces - oe.get(2)).max() < 1e-8
         assert np.abs(eng.positions - oe.get(0)).max() < 1e-9
+
+
+@pytest.mark.parametrize("profile", ["ref", "phys"])
+def test_fp64_pairs_half_a_box_apart(oracle, profile):
+    """Lattice sites exactly half a box apart in a box narrower than twice the
+    cutoff: the reference rounds the image halfway from zero, and so does the
+    FP64 path (the other image would turn the force round).  Every second site is
+    displaced, so that the forces do not cancel.  Tolerance: 1e-9."""
+    g = np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    w = W.lj_fluid(64, 0.7, 1.0, 3)
+    w.box, w.lj_cutoff = 2.0, 1.05
+    w.pos = 0.5 * g + 0.02 * np.random.default_rng(2).random((64, 3)) * (g.sum(1) % 2)[:, None]
+    c = w.config()
+    f, _ = _engine(c, "fp64", profile).compute_forces()
+    f_o, _ = oracle.forces(c, profile)
+    assert rel_rms(f, f_o) < 1e-9
