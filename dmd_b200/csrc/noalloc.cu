@@ -85,7 +85,10 @@ namespace {
 std::mutex g_mu;
 void* g_addr[64] = {};  // device address of g_nb_scratch per device ordinal
 
-// Per-device set-up: with the device current, resolve the array's address once.
+// Per-device set-up: with the device current, resolve the array's address and
+// set the pair kernels' attributes once (the FP64 kernel's shared memory needs
+// one to be launched at all; a caller of this entry need not have made an
+// engine).  Neither allocates.
 // The address is cached per device ordinal, so calls must run in the device's
 // primary context (the runtime API's default); a caller that switches to
 // another context on the same device, or resets the device, would be handed
@@ -96,6 +99,10 @@ int scratch_address(int dev, unsigned char** out) {
     if (!g_addr[dev]) {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_nb_scratch) != cudaSuccess || !p) return DMDGPU_ERR_GPU;
+        if (!configure_nonbonded_kernels()) {
+            cudaGetLastError();  // reported by the status, not left pending
+            return DMDGPU_ERR_GPU;
+        }
         g_addr[dev] = p;
     }
     *out = static_cast<unsigned char*>(g_addr[dev]);

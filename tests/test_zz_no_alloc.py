@@ -132,3 +132,30 @@ def test_noalloc_reports_list_overflow():
     pos_s = np.stack([small.pos_x, small.pos_y, small.pos_z], 1)
     F, _ = _noalloc(small, pos_s, "phys", "mixed")
     assert np.all(np.isfinite(F))
+
+
+@pytest.mark.parametrize("profile", ["phys", "ref"])
+def test_noalloc_fp64_without_an_engine(oracle, profile, tmp_path):
+    """The FP64 call in a process of its own that makes no engine: nothing but
+    the call itself prepares the device for its kernels.  Against the oracle's
+    Lennard-Jones and real-space Coulomb components."""
+    import os
+    import subprocess
+    import sys
+    cfg = W.water_box(n_mol=500, box=(500 / 33.43) ** (1 / 3), seed=21, spacing=0.1).config()
+    pos = np.stack([cfg.pos_x, cfg.pos_y, cfg.pos_z], 1)
+    out = tmp_path / "f.npz"
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = (f"import sys; sys.path[:0] = [{here!r}, {os.path.dirname(here)!r}]\n"
+            "import numpy as np, test_zz_no_alloc as t\n"
+            "c = t.W.water_box(n_mol=500, box=(500 / 33.43) ** (1 / 3), seed=21, spacing=0.1).config()\n"
+            f"F, e = t._noalloc(c, np.stack([c.pos_x, c.pos_y, c.pos_z], 1), {profile!r}, 'fp64')\n"
+            f"np.savez({str(out)!r}, F=F, e=e)\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    got = np.load(out)
+    f0, e0, _ = oracle.component(cfg, profile, 0, pos=pos)
+    f4, e4, _ = oracle.component(cfg, profile, 4, pos=pos)
+    err = np.linalg.norm(got["F"] - (f0 + f4)) / np.linalg.norm(f0 + f4)
+    assert err < TOL["fp64"], err
+    assert abs(float(got["e"]) - (e0 + e4)) <= 10 * TOL["fp64"] * max(abs(e0 + e4), 1.0)
