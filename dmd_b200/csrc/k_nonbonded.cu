@@ -877,6 +877,10 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
     if (COUL && lane < EWALD_N) S.cf[lane] = d.ewald_poly[EWALD_N * r + lane];
     const uint32_t rot = rotated_columns(mk, lane);
     const uint32_t col = __funnelshift_l(rot, rot, lane);  // bit j: (lane, entry j) interacts
+    // A pair of an atom with a non-finite coordinate passes no distance test.  It is
+    // listed all the same: its force is then not a number, which is what reports it.
+    const bool odd_i = !isfinite(xi.x + xi.y + xi.z), odd_j = !isfinite(xj.x + xj.y + xj.z);
+    const uint32_t odd = __ballot_sync(FULL, odd_j) | (odd_i ? FULL : 0u);
     __syncwarp();
     const bool has_lj = (R.flags & F_LJ) != 0;
     const double rl2 = has_lj ? R.rc_lj2 : 0.0, rcc2 = COUL ? R.rc_c2 : 0.0;
@@ -924,7 +928,7 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
         __syncwarp();  // the staged entries have been read
         return false;
     }
-    nm &= col;
+    nm = (nm | odd) & col;
     const uint32_t below = (1u << lane) - 1u;
     const double us = COUL ? 2.0 / R.rc_c2 : 0.0;
     const double2* lj = d.lj64 + R.lj_off;

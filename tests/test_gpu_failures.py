@@ -103,3 +103,21 @@ def test_corrupt_checkpoints_refused(tmp_path):
     fresh = _engine(cfg, "fp64", "ref")
     fresh.load_checkpoint(str(good))
     assert fresh.current_step == 4
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("profile", ["phys", "ref"])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_non_finite_velocity_reported_without_charges(precision, profile, value):
+    """One atom of a Lennard-Jones fluid with a non-finite velocity: its position
+    is non-finite after the drift, no other component than the pair forces sees
+    it, and the step that evaluates them reports it."""
+    from dmd_b200.core import DmdGpuError
+    eng = _engine(W.lj_fluid(500, 0.8, 1.0, 3).config(), precision, profile)
+    eng.run_n(2)
+    vel = eng.velocities
+    vel[17, 1] = value
+    eng.set_velocities(vel)
+    with pytest.raises(DmdGpuError) as ei:
+        eng.run_n(1)
+    assert ei.value.code == ERR_NAN, str(ei.value)
