@@ -65,6 +65,10 @@ struct HostRep {
     bool done = false;
     bool polled = false;
     bool on_device = false;    // packed into the current device table (its state lives there)
+    // FP64, real-space Coulomb: coefficients of its Ewald polynomial (none where 24 do
+    // not reach rounding), found once: alpha and the cutoff do not change
+    std::vector<double> ewald;
+    bool ewald_known = false;
 };
 
 // Device memory of the packed table: slabs kept by the batch across table
@@ -151,6 +155,7 @@ class Batch {
   private:
     int check_cuda(cudaError_t e, const char* what);
     int build_host(HostRep& hr, unsigned comp_mask);
+    void fit_ewald(HostRep& h);
     void enqueue_eval(int pass);
     void enqueue_rebuild();
     void enqueue_step(bool first, bool begun = false, int next = 0);

@@ -267,3 +267,65 @@ def test_fp64_pairs_half_a_box_apart(oracle, profile):
     f, _ = _engine(c, "fp64", profile).compute_forces()
     f_o, _ = oracle.forces(c, profile)
     assert rel_rms(f, f_o) < 1e-9
+
+
+def test_fp64_tables_change_without_refitting():
+    """Admitting and releasing one FP64 replica beside 48 charged ones fits no Ewald
+    polynomial again: it takes about as long as with an alpha beyond the
+    polynomial's reach, which is refused at once (48 fits, twice, are 24 ms or
+    more; best of nine, 8 ms apart at most)."""
+    import time
+    from dmd_b200.batch import Batch
+
+    def change(alpha):
+        cfgs = [W.water_box(n_mol=60 + k, box=((60 + k) / 33.43) ** (1 / 3) + 1.2, seed=k, spacing=0.3).config()
+                for k in range(48)]
+        for c in cfgs:
+            c.ewald_coeff = alpha
+        b = Batch(precision="fp64", profile="phys")
+        for c in cfgs:
+            b.admit(c, 1 << 40)
+        b.step(1)
+        best = math.inf
+        for _ in range(9):
+            t = time.perf_counter()
+            k = b.admit(cfgs[0], 1 << 40)
+            b.step(1)
+            b.release(k)
+            b.step(1)
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    assert change(3.12) < change(9.0) + 0.008
+
+
+def test_fp64_ewald_polynomials_of_one_table(oracle):
+    """Replicas of one FP64 table that share a polynomial, have one of their own (alpha
+    or cutoff) or none (alpha rc 4.2), admitted at different times and into a
+    released slot: each has the forces it has alone, bit for bit, and the oracle's
+    (1e-9)."""
+    from dmd_b200.batch import Batch
+
+    def make(k, alpha, rc):
+        c = W.water_box(n_mol=429, box=2.34, seed=k, spacing=0.117).config()
+        c.ewald_coeff, c.lj_cutoff, c.coulomb_cutoff = alpha, rc, rc
+        return c
+
+    kinds = [(3.12, 1.0), (3.12, 1.0), (2.9, 1.0), (3.12, 0.9), (4.2, 1.0), (3.12, 1.0)]
+    cfgs = [make(k, a, rc) for k, (a, rc) in enumerate(kinds)]
+    b = Batch(precision="fp64", profile="phys")
+    first = b.admit(make(9, 3.0, 1.0), 1 << 40)
+    slots = [b.admit(c, 1 << 40) for c in cfgs[:3]]
+    b.step(1)
+    b.release(first)
+    slots += [b.admit(c, 1 << 40) for c in cfgs[3:]]
+    b.step(1)
+    for k, (c, slot) in enumerate(zip(cfgs, slots)):
+        n = 2 if k < 3 else 1
+        eng = _engine(c, "fp64", "phys")
+        for _ in range(n):
+            eng.run_n(1)
+            if n == 2 and _ == 0:
+                eng.repack()
+        assert np.array_equal(b.forces(slot), eng.forces) and np.array_equal(b.positions(slot), eng.positions)
+        assert rel_rms(eng.forces, oracle.forces(c, "phys", pos=eng.positions)[0]) < 1e-9
