@@ -2217,9 +2217,9 @@ void Batch::launch_info(dmdgpu_launch_info* out) const {
     out->packed = packed_ && !order_.empty() ? 1 : 0;
     if (!out->packed) return;
     out->nb_form = nb_form_ == NB_CLUSTER8 ? DMDGPU_NB_CLUSTER8 : DMDGPU_NB_CHUNK32;
-    out->nb_blocks_per_sm = fp64_ ? 8 : nb_blocks_per_sm_;
+    out->nb_blocks_per_sm = fp64_ ? NB64_BLOCKS_PER_SM : nb_blocks_per_sm_;
     out->tuned = tuned_ ? 1 : 0;
-    out->min_image_kernel = fp64_ ? 0 : dev_.mi_split;  // the FP64 kernel always takes it
+    out->min_image_kernel = fp64_ ? 0 : dev_.mi_split;  // the FP64 kernel has both forms in one
     out->n_replicas = static_cast<int32_t>(order_.size());
     out->n_atoms = dev_.n_atoms;
     out->launches_per_step = per_step_launches_;

@@ -1087,9 +1087,8 @@ __device__ __noinline__ bool nb_chunk_f64_energy(const Dev& d, const Rep& R, Rep
 }
 
 // Persistent, chunks claimed as in k_nb_f32 (first chunk without a claim).
-// 2 blocks of 256 threads per SM, by registers and by shared memory.
 template <bool PHYS>
-__global__ void __launch_bounds__(256, 2) k_nb_f64(const __grid_constant__ Dev d) {
+__global__ void __launch_bounds__(256, NB64_BLOCKS_PER_SM) k_nb_f64(const __grid_constant__ Dev d) {
     chain_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -1189,8 +1188,8 @@ bool configure_nonbonded_kernels() {
 void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_per_sm, int form,
                       cudaStream_t st, long long* nlaunch) {
     if (fp64) {
-        if (phys) launch_chained_smem(k_nb_f64<true>, n_sm * 2, 256, NB64_SMEM, st, d);
-        else launch_chained_smem(k_nb_f64<false>, n_sm * 2, 256, NB64_SMEM, st, d);
+        if (phys) launch_chained_smem(k_nb_f64<true>, n_sm * NB64_BLOCKS_PER_SM, 256, NB64_SMEM, st, d);
+        else launch_chained_smem(k_nb_f64<false>, n_sm * NB64_BLOCKS_PER_SM, 256, NB64_SMEM, st, d);
     } else {
         const bool ljs = d.n_lj <= LJ_SMEM;
         // a table without real-space Coulomb runs the LJ-only instantiation

@@ -48,6 +48,9 @@ void launch_rebuild(const Dev& d, const int* bin_rep, int n_sm, bool chained, cu
 // single system with a PME chain timing the other shapes too.  Results do not
 // depend on the launch shape (one warp per work item, fixed-point sums).
 enum NbForm { NB_CHUNK32 = 0, NB_CLUSTER8 = 1 };
+// The FP64 kernel's blocks per SM, whatever blocks_per_sm says: what its registers
+// and its shared memory allow.
+constexpr int NB64_BLOCKS_PER_SM = 2;
 void launch_nonbonded(const Dev& d, bool fp64, bool phys, int n_sm, int blocks_per_sm, int form,
                       cudaStream_t st, long long* nlaunch);
 // Whether a kernel function (cudaGraphKernelNodeGetParams' func) is one of the

@@ -233,9 +233,10 @@ typedef struct dmdgpu_launch_info {
     int32_t nb_form;           /* DMDGPU_NB_CHUNK32 or DMDGPU_NB_CLUSTER8 (FP64: CHUNK32) */
     int32_t nb_blocks_per_sm;  /* persistent pair-kernel blocks per SM */
     int32_t tuned;             /* 1: blocks per SM measured (now or cached) for this kind
-                                  of table; 0: from the list's size */
+                                  of table, or fixed (FP64); 0: from the list's size */
     int32_t min_image_kernel;  /* 1: boxes narrower than twice the list cutoff (or under
-                                  a barostat) also run the minimum-image pair kernel */
+                                  a barostat) also run the minimum-image pair kernel
+                                  (FP64: 0, its one kernel takes either image) */
     int32_t n_replicas;
     int64_t n_atoms;
     int64_t launches_per_step; /* kernels in one captured step */

@@ -329,3 +329,13 @@ def test_fp64_ewald_polynomials_of_one_table(oracle):
                 eng.repack()
         assert np.array_equal(b.forces(slot), eng.forces) and np.array_equal(b.positions(slot), eng.positions)
         assert rel_rms(eng.forces, oracle.forces(c, "phys", pos=eng.positions)[0]) < 1e-9
+
+
+def test_launch_info_of_the_fp64_path():
+    """FP64 tables report the two blocks per SM that their pair kernel is launched
+    with, whatever the list's size."""
+    for n in (500, 20000):
+        eng = _engine(W.lj_fluid(n, 0.8, 1.0, 3).config(), "fp64", "phys")
+        eng.run_n(1)
+        info = eng.launch_info()
+        assert info["nb_blocks_per_sm"] == 2 and info["nb_form"] == "chunk32" and not info["min_image_kernel"]
