@@ -2058,17 +2058,82 @@ void Batch::record(cudaEvent_t e, cudaStream_t st) {
     else cudaEventRecord(e, st);
 }
 
+// A copy of the one-step graph with event record nodes around every pair-kernel
+// launch and every PME chain.  g (whose nodes name ge's event nodes) lives as
+// long as ge.
+struct Batch::TimedStep {
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t ge = nullptr;
+    std::vector<cudaGraphNode_t> nb, pme;  // start, end, start, end, ...
+    long long launches = 0;                // kernels of the step
+    ~TimedStep() {
+        if (ge) cudaGraphExecDestroy(ge);
+        if (g) cudaGraphDestroy(g);
+    }
+};
+
+int Batch::capture_timed(bool first, TimedStep* t) {
+    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> nb0, pme0;
+    prof_nb_ = &nb0;
+    prof_pme_ = &pme0;
+    const long long before = launches_;
+    cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        enqueue_step(first);
+        e = cudaStreamEndCapture(stream_, &t->g);
+    }
+    prof_nb_ = nullptr;
+    prof_pme_ = nullptr;
+    t->launches = launches_ - before;
+    launches_ = before;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        t->g = nullptr;
+        return fail(DMDGPU_ERR_GPU, std::string("timed capture failed: ") + cudaGetErrorString(e));
+    }
+    // the event record nodes, in the order of nb0 / pme0 (start, end)
+    t->nb.assign(2 * nb0.size(), nullptr);
+    t->pme.assign(2 * pme0.size(), nullptr);
+    size_t nn = 0;
+    cudaGraphGetNodes(t->g, nullptr, &nn);
+    std::vector<cudaGraphNode_t> nodes(nn);
+    cudaGraphGetNodes(t->g, nodes.data(), &nn);
+    for (cudaGraphNode_t node : nodes) {
+        cudaGraphNodeType type;
+        if (cudaGraphNodeGetType(node, &type) != cudaSuccess || type != cudaGraphNodeTypeEventRecord) continue;
+        cudaEvent_t ev = nullptr;
+        if (cudaGraphEventRecordNodeGetEvent(node, &ev) != cudaSuccess) continue;
+        for (size_t k = 0; k < nb0.size(); ++k) {
+            if (ev == nb0[k].first) t->nb[2 * k] = node;
+            if (ev == nb0[k].second) t->nb[2 * k + 1] = node;
+        }
+        for (size_t k = 0; k < pme0.size(); ++k) {
+            if (ev == pme0[k].first) t->pme[2 * k] = node;
+            if (ev == pme0[k].second) t->pme[2 * k + 1] = node;
+        }
+    }
+    for (cudaGraphNode_t node : t->nb)
+        if (!node) return fail(DMDGPU_ERR_GPU, "timed capture: pair-kernel event nodes not found");
+    for (cudaGraphNode_t node : t->pme)
+        if (!node) return fail(DMDGPU_ERR_GPU, "timed capture: PME event nodes not found");
+    set_node_priorities(t->g);
+    return check_cuda(cudaGraphInstantiate(&t->ge, t->g, cudaGraphInstantiateFlagUseNodePriority), "cudaGraphInstantiate");
+}
+
 // n steps with device timing.  Every step is one launch of a one-step graph,
 // between two events recorded on the main stream (the optional L2 flush goes
-// before the first event).  Seven of every eight launches are of the step
-// graph run_n uses; every eighth is of a copy with event record nodes around
-// every pair-kernel launch and every PME chain, whose nodes are pointed at
-// fresh events before each launch (cudaGraphExecEventRecordNodeSetEvent), so
-// the pair kernel's and the PME chain's durations are those of the sampled
-// steps.  Event nodes on the critical path add a few microseconds to their
-// step, and capturing all n steps into one graph with their events changed
-// how the branches were scheduled (water 30k: a step period of ~143 us
-// against ~124 us for run_n's graph), hence one step graph and sampling.
+// before the first event).  Seven of every eight launches are of the one-step
+// graph run_n would launch there (REF: with or without the first evaluation, by
+// the list cadence; several steps per graph, which run_n takes once a table
+// has run for a while, have no place for events between them); every eighth is
+// of a copy with event record nodes around every pair-kernel launch and every
+// PME chain, whose nodes are pointed at fresh events before each launch
+// (cudaGraphExecEventRecordNodeSetEvent), so the pair kernel's and the PME
+// chain's durations are those of the sampled steps.  Event nodes on the
+// critical path add a few microseconds to their step, and capturing all n
+// steps into one graph with their events changed how the branches were
+// scheduled (water 30k: a step period of ~143 us against ~124 us for run_n's
+// graph), hence one step per graph and sampling.
 int Batch::step_timed(int n, long long flush_bytes, dmdgpu_timing* out) {
     st_fresh_ = sim_ok_ = false;  // device work follows: the host mirror is stale
     CK(cudaSetDevice(device_));
@@ -2093,105 +2158,62 @@ int Batch::step_timed(int n, long long flush_bytes, dmdgpu_timing* out) {
         CK(cudaMalloc(&flush_buf_, flush_bytes));
         flush_bytes_ = flush_bytes;
     }
+    const bool skip = skip_first();
+    if (skip) {
+        const int rc = load_cadence();
+        if (rc) return rc;
+        st_fresh_ = sim_ok_ = false;
+    }
     if (fp64_) launch_mark_read(dev_, n, stream_, &launches_);
-    // capture one step with its pair-kernel and PME events
     ev_used_ = 0;
-    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> nb0, pme0;
-    prof_nb_ = &nb0;
-    prof_pme_ = &pme0;
-    cudaGraph_t g;
-    const long long before = launches_;
-    capture_error_ = false;
-    cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        enqueue_step(need_eval1_);
-        e = cudaStreamEndCapture(stream_, &g);
+    TimedStep sample[2];  // [1]: the step without its first evaluation
+    for (int k = 0; k < (skip ? 2 : 1); ++k) {
+        const int rc = capture_timed(k == 0 && need_eval1_, &sample[k]);
+        if (rc) return rc;
     }
-    prof_nb_ = nullptr;
-    prof_pme_ = nullptr;
-    if (e != cudaSuccess || capture_error_) {
-        cudaGetLastError();
-        return fail(DMDGPU_ERR_GPU, std::string("timed capture failed: ") + cudaGetErrorString(e));
-    }
-    const long long per_step = launches_ - before;
-    launches_ = before;
-    // the event record nodes, in the order of nb0 / pme0 (start, end)
-    std::vector<cudaGraphNode_t> nb_nodes(2 * nb0.size()), pme_nodes(2 * pme0.size());
-    {
-        size_t nn = 0;
-        cudaGraphGetNodes(g, nullptr, &nn);
-        std::vector<cudaGraphNode_t> nodes(nn);
-        cudaGraphGetNodes(g, nodes.data(), &nn);
-        for (cudaGraphNode_t node : nodes) {
-            cudaGraphNodeType t;
-            if (cudaGraphNodeGetType(node, &t) != cudaSuccess || t != cudaGraphNodeTypeEventRecord) continue;
-            cudaEvent_t ev = nullptr;
-            if (cudaGraphEventRecordNodeGetEvent(node, &ev) != cudaSuccess) continue;
-            for (size_t k = 0; k < nb0.size(); ++k) {
-                if (ev == nb0[k].first) nb_nodes[2 * k] = node;
-                if (ev == nb0[k].second) nb_nodes[2 * k + 1] = node;
-            }
-            for (size_t k = 0; k < pme0.size(); ++k) {
-                if (ev == pme0[k].first) pme_nodes[2 * k] = node;
-                if (ev == pme0[k].second) pme_nodes[2 * k + 1] = node;
-            }
-        }
-        for (cudaGraphNode_t node : nb_nodes)
-            if (!node) {
-                cudaGraphDestroy(g);
-                return fail(DMDGPU_ERR_GPU, "timed capture: pair-kernel event nodes not found");
-            }
-        for (cudaGraphNode_t node : pme_nodes)
-            if (!node) {
-                cudaGraphDestroy(g);
-                return fail(DMDGPU_ERR_GPU, "timed capture: PME event nodes not found");
-            }
-    }
-    set_node_priorities(g);
-    cudaGraphExec_t ge;
-    e = cudaGraphInstantiate(&ge, g, cudaGraphInstantiateFlagUseNodePriority);
-    if (e != cudaSuccess) {
-        cudaGraphDestroy(g);
-        return check_cuda(e, "cudaGraphInstantiate");
-    }
-    // g (whose nodes name the exec graph's event nodes) lives until the end
     // events for every launch: the step's pair, then the nodes' pairs
-    const size_t per_launch = 2 + nb_nodes.size() + pme_nodes.size();
-    const size_t need = ev_used_ + per_launch * static_cast<size_t>(n);
+    const size_t need = ev_used_ + (2 + sample[0].nb.size() + sample[0].pme.size()) * static_cast<size_t>(n);
     while (ev_pool_.size() < need) {
         cudaEvent_t ev;
         CK(cudaEventCreate(&ev));
         ev_pool_.push_back(ev);
     }
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> nb, pme, steps;
-    auto point = [&](const std::vector<cudaGraphNode_t>& nodes, std::vector<std::pair<cudaEvent_t, cudaEvent_t>>& out) {
+    cudaError_t e = cudaSuccess;
+    auto point = [&](const TimedStep& t, const std::vector<cudaGraphNode_t>& nodes,
+                     std::vector<std::pair<cudaEvent_t, cudaEvent_t>>& to) {
         for (size_t k = 0; k < nodes.size() && e == cudaSuccess; k += 2) {
             const cudaEvent_t x = next_event(), y = next_event();
-            e = cudaGraphExecEventRecordNodeSetEvent(ge, nodes[k], x);
-            if (e == cudaSuccess) e = cudaGraphExecEventRecordNodeSetEvent(ge, nodes[k + 1], y);
-            out.emplace_back(x, y);
+            e = cudaGraphExecEventRecordNodeSetEvent(t.ge, nodes[k], x);
+            if (e == cudaSuccess) e = cudaGraphExecEventRecordNodeSetEvent(t.ge, nodes[k + 1], y);
+            to.emplace_back(x, y);
         }
     };
+    long long n_sampled = 0, n_kernels = 0;
     for (int i = 0; i < n && e == cudaSuccess; ++i) {
         if (flush_buf_) cudaMemsetAsync(flush_buf_, i & 0xff, flush_bytes_, stream_);
+        const bool first = !skip || cadence_due();
+        TimedStep& t = sample[first ? 0 : 1];
         const cudaEvent_t a = next_event(), b = next_event();
         const bool sampled = (i % 8) == 7 || (n < 8 && i == n - 1);
         if (sampled) {
-            point(nb_nodes, nb);
-            point(pme_nodes, pme);
+            point(t, t.nb, nb);
+            point(t, t.pme, pme);
             if (e != cudaSuccess) break;
+            ++n_sampled;
         }
         cudaEventRecord(a, stream_);
-        e = cudaGraphLaunch(sampled ? ge : graph_, stream_);
+        e = cudaGraphLaunch(sampled ? t.ge : (first ? graph_ : graph_skip_), stream_);
         cudaEventRecord(b, stream_);
         steps.emplace_back(a, b);
-        launches_ += per_step;
+        n_kernels += t.launches;
+        if (skip) advance_cadence(first);
     }
+    launches_ += n_kernels;
     const cudaError_t e_sync = cudaStreamSynchronize(stream_);
     if (e == cudaSuccess) e = e_sync;
-    cudaGraphExecDestroy(ge);
-    cudaGraphDestroy(g);
     if (e != cudaSuccess) return check_cuda(e, "timed steps");
+    sim_ok_ = skip;
     float ms = 0.f;
     for (auto& pr : steps) {
         CK(cudaEventElapsedTime(&ms, pr.first, pr.second));
@@ -2206,9 +2228,9 @@ int Batch::step_timed(int n, long long flush_bytes, dmdgpu_timing* out) {
         out->pme_ms += ms;
     }
     out->nonbonded_launches = static_cast<long long>(nb.size());
-    out->sampled_steps = static_cast<long long>(nb_nodes.empty() ? 0 : nb.size() / (nb_nodes.size() / 2));
+    out->sampled_steps = n_sampled;
     int rc = sync_status();
-    out->kernel_launches = per_step * n;
+    out->kernel_launches = n_kernels;
     return rc;
 }
 

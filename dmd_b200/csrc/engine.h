@@ -186,7 +186,6 @@ class Batch {
     // bonded terms on a third stream, beside both
     cudaStream_t bond_stream_ = nullptr;
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr, ev_join_b_ = nullptr;
-    bool capture_error_ = false;
     std::vector<std::unique_ptr<HostRep>> reps_;   // indexed by slot (nullptr = free)
     std::vector<int> order_;                        // packed replica index -> slot
     SlabStore slabs_;                                // declared before arena_: outlives it
@@ -214,6 +213,8 @@ class Batch {
     bool joined_ = false;                   // the last evaluation joined other streams
     long long steps_run_ = 0;               // steps launched from graph_ or graph_many_
     int capture_steps(int n, bool first, cudaGraphExec_t* out);
+    struct TimedStep;
+    int capture_timed(bool first, TimedStep* t);
     // REF list cadence per packed replica, followed on the host (run_steps)
     struct Cadence {
         long long left;  // steps to the replica's target

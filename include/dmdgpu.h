@@ -255,9 +255,11 @@ typedef struct dmdgpu_timing {
     int64_t sampled_steps;     /* steps whose pair-kernel and PME launches were timed */
 } dmdgpu_timing;
 
-/* dmdgpu_step with device timing: the step graph (the one dmdgpu_step launches,
- * with event records around every non-bonded launch and every PME chain) is
- * launched n times, each launch between two events on the context's stream.
+/* dmdgpu_step with device timing: n launches of the one-step graph that
+ * dmdgpu_step launches (REF: with the first evaluation only in the steps whose
+ * list cadence needs it), each between two events on the context's stream; every
+ * eighth is of a copy with event records around every non-bonded launch and
+ * every PME chain.
  * When l2_flush_bytes > 0 a buffer of that size is overwritten between steps
  * (outside the timed intervals) so each step starts with a cold L2.  Not
  * available for a REF Andersen thermostat (its random stream is drawn on the

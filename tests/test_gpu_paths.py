@@ -339,3 +339,19 @@ def test_launch_info_of_the_fp64_path():
         eng.run_n(1)
         info = eng.launch_info()
         assert info["nb_blocks_per_sm"] == 2 and info["nb_form"] == "chunk32" and not info["min_image_kernel"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("start", [5, 7])
+def test_timed_ref_steps_are_the_steps_that_run(precision, start):
+    """REF: timed steps issue a first evaluation where run_n does, from any point of
+    the list cadence, and leave the state and the cadence that run_n leaves."""
+    a, b = _engine(_argon(4), precision, "ref"), _engine(_argon(4), precision, "ref")
+    a.run_n(start), b.run_n(start)
+    n0 = a.kernel_launches()
+    a.run_n(20)
+    n1 = a.kernel_launches()
+    t = b.step_timed(20, 0)
+    assert t["kernel_launches"] == n1 - n0 - (precision == "fp64")  # less the mark of the step that is read
+    a.run_n(7), b.run_n(7)
+    assert np.array_equal(a.positions, b.positions) and np.array_equal(a.velocities, b.velocities)
