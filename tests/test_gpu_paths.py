@@ -355,3 +355,110 @@ def test_timed_ref_steps_are_the_steps_that_run(precision, start):
     assert t["kernel_launches"] == n1 - n0 - (precision == "fp64")  # less the mark of the step that is read
     a.run_n(7), b.run_n(7)
     assert np.array_equal(a.positions, b.positions) and np.array_equal(a.velocities, b.velocities)
+
+
+def _long_cases():
+    def lj(thermostat="none"):
+        return _set(W.lj_fluid(500, 0.8, 1.0, 3).config(), thermostat)
+
+    def water(barostat="none"):
+        c = W.water_box(n_mol=430, box=(430 / 33.43) ** (1 / 3), seed=5, spacing=0.1).config()
+        return _set(c, "nose-hoover", barostat)
+
+    return {"lj": (lj, "mixed", "phys"), "lj-nh": (lambda: lj("nose-hoover"), "mixed", "phys"),
+            "lj-andersen": (lambda: lj("andersen"), "mixed", "phys"),
+            "lj-fp64": (lambda: lj("berendsen"), "fp64", "phys"),
+            "water": (water, "mixed", "phys"), "water-fp64": (water, "fp64", "phys"),
+            "water-npt": (lambda: water("berendsen"), "mixed", "phys"),
+            "rigid": (lambda: _rigid_water(430, "tri"), "mixed", "phys"),
+            "argon-ref": (lambda: _argon(4), "mixed", "ref"), "argon-ref-fp64": (lambda: _argon(4), "fp64", "ref"),
+            "argon-ref-npt": (lambda: _set(_argon(4), "berendsen", "berendsen"), "mixed", "ref")}
+
+
+def _set(c, thermostat, barostat="none"):
+    c.thermostat.type, c.barostat.type = thermostat, barostat
+    if thermostat != "none":
+        c.thermostat.temperature = 120.0
+    return c
+
+
+@pytest.mark.parametrize("case", list(_long_cases()))
+def test_several_steps_per_launch(case):
+    """Tables that keep running take four steps (REF: the five of a list cadence) per
+    graph once 256 have run.  Calls of mixed length beyond that point leave the
+    state, bit for bit, that calls of three steps leave, which never do."""
+    make, precision, profile = _long_cases()[case]
+    a, b = _engine(make(), precision, profile), _engine(make(), precision, profile)
+    a.run_n(260)
+    for n in (9, 4, 1, 7, 3, 16, 5):
+        a.run_n(n)
+    for _ in range(101):
+        b.run_n(3)
+    b.run_n(2)
+    if precision == "mixed" and case != "argon-ref-npt":
+        # the later steps of a graph begin in the update of the one before: fewer launches
+        assert a.kernel_launches() < b.kernel_launches()
+    assert np.array_equal(a.positions, b.positions) and np.array_equal(a.velocities, b.velocities)
+    assert np.array_equal(a.forces, b.forces)
+    sa, sb = a.scalars(), b.scalars()
+    assert (sa.step, sa.time, sa.box) == (sb.step, sb.time, sb.box)
+    assert (sa.kinetic_energy, list(sa.e_terms)) == (sb.kinetic_energy, list(sb.e_terms))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("profile", ["phys", "ref"])
+def test_targets_inside_a_launch_of_several_steps(profile, precision):
+    """Replicas that reach their targets inside a graph of several steps stop there,
+    with their energies, while the others go on: bit for bit as in calls of three."""
+    from dmd_b200.batch import Batch
+    cfgs = [_argon(3 + k % 2, k) if profile == "ref" else _set(W.lj_fluid(400 + 90 * k, 0.8, 1.0, k).config(), th)
+            for k, th in enumerate(("none", "berendsen", "nose-hoover", "none", "berendsen"))]
+    targets = [261, 266, 279, 303, 1000]
+    out = []
+    for calls in ((260, 45), (3,) * 101 + (2,)):
+        b = Batch(precision=precision, profile=profile)
+        slots = [b.admit(c, n) for c, n in zip(cfgs, targets)]
+        for n in calls:
+            b.step(n)
+        out.append([(b.scalars(k).step, b.scalars(k).kinetic_energy, list(b.scalars(k).e_terms[:]) if n < 1000 else None,
+                     b.positions(k).tobytes(), b.velocities(k).tobytes()) for k, n in zip(slots, targets)])
+    assert [o[0] for o in out[0]] == [261, 266, 279, 303, 305]
+    assert out[0] == out[1]
+
+
+def _same_energies(e, e_o, tol):
+    for k in ("lj", "coul_real", "coul_recip", "total"):
+        got = sum(e.values()) if k == "total" else e[k]
+        assert abs(got - e_o[k]) <= 10 * tol * max(abs(e_o[k]), 1.0), (k, got, e_o[k])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_mol,spacing", [(130, 0.2), (400, 0.105), (400, 0.022)])
+def test_pme_mesh_energies(oracle, n_mol, spacing, precision):
+    """Energies on the meshes of test_pme_mesh_sizes, term by term (single-point
+    tolerances)."""
+    box = (n_mol / 33.43) ** (1 / 3)
+    c = W.water_box(n_mol=n_mol, box=box, seed=9, spacing=spacing).config()
+    _, e = _engine(c, precision, "phys").compute_forces()
+    _same_energies(e, oracle.forces(c, "phys")[1], {"fp64": 1e-9, "mixed": 1e-5}[precision])
+
+
+@pytest.mark.parametrize("alpha", [3.12, 4.2])
+@pytest.mark.parametrize("rc_lj", [1.0, 0.85])
+@pytest.mark.parametrize("n_mol", [110, 429])
+def test_fp64_pair_energies(oracle, n_mol, rc_lj, alpha):
+    """Energies and the virial of the pair forms of test_fp64_pair_forms: of a single
+    point, and of the evaluation that ends a run (1e-7: the positions there agree to
+    1e-10 nm or better, on forces of up to 1e4)."""
+    box = (n_mol / 33.43) ** (1 / 3)
+    c = W.water_box(n_mol=n_mol, box=box, seed=5, spacing=box / round(box / 0.1)).config()
+    c.lj_cutoff, c.ewald_coeff = rc_lj, alpha
+    eng = _engine(c, "fp64", "phys")
+    _same_energies(eng.compute_forces()[1], oracle.forces(c, "phys")[1], 1e-9)
+    oe = oracle.engine(c, "phys")
+    oe.step(5)
+    run = _engine(c, "fp64", "phys")
+    run.run_n(5)
+    e_o = oe.energy()
+    _same_energies(run.energy_terms(), e_o, 1e-8)
+    assert abs(run.scalars().virial - e_o["virial"]) <= 1e-7 * abs(e_o["virial"])
