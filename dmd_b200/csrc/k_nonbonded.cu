@@ -793,6 +793,12 @@ __device__ __noinline__ void nb_chunk_f64_erfc(const Dev& d, const Rep& R, RepSt
     __syncwarp();
 }
 
+// x in single precision, an infinite one as not a number.
+__device__ __forceinline__ float finite_or_nan(double x) {
+    const float f = static_cast<float>(x);
+    return f + (f - f);
+}
+
 // 1 / sqrt(x), x > 0: the single-precision approximation and one Halley step
 // (cubic: its ~2^-22 relative error becomes ~2^-65, below rounding).
 __device__ __forceinline__ double rsqrt_h(double x) {
@@ -873,14 +879,10 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
     S.tj[lane] = tj;
     S.js[lane] = js;
     if (!MI)
-        S.jf[lane] = make_float4(static_cast<float>(xj.x), static_cast<float>(xj.y), static_cast<float>(xj.z), 0.f);
+        S.jf[lane] = make_float4(finite_or_nan(xj.x), finite_or_nan(xj.y), finite_or_nan(xj.z), 0.f);
     if (COUL && lane < EWALD_N) S.cf[lane] = d.ewald_poly[EWALD_N * r + lane];
     const uint32_t rot = rotated_columns(mk, lane);
     const uint32_t col = __funnelshift_l(rot, rot, lane);  // bit j: (lane, entry j) interacts
-    // A pair of an atom with a non-finite coordinate passes no distance test.  It is
-    // listed all the same: its force is then not a number, which is what reports it.
-    const bool odd_i = !isfinite(xi.x + xi.y + xi.z), odd_j = !isfinite(xj.x + xj.y + xj.z);
-    const uint32_t odd = __ballot_sync(FULL, odd_j) | (odd_i ? FULL : 0u);
     __syncwarp();
     const bool has_lj = (R.flags & F_LJ) != 0;
     const double rl2 = has_lj ? R.rc_lj2 : 0.0, rcc2 = COUL ? R.rc_c2 : 0.0;
@@ -892,9 +894,10 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
     // that no pair inside can exceed: with u = 2^-24, a component of the
     // difference is off by at most 2 u (|x_i| + rmax) = err, r^2 by 2 sqrt(3)
     // rmax err + 3 err^2 and 4 u of itself.
-    // The same for half a box (hl2), from below.
+    // The same for half a box (hl2), from below.  A distance that is not a number
+    // passes: the pair's force is then not a number either, which reports it.
     float thr = 0.f, hl2 = 0.f;
-    const float xf = static_cast<float>(xi.x), yf = static_cast<float>(xi.y), zf = static_cast<float>(xi.z);
+    const float xf = finite_or_nan(xi.x), yf = finite_or_nan(xi.y), zf = finite_or_nan(xi.z);
     if (!MI) {
         const double rmax = sqrt(rmax2);
         const double xmax = fmax(fmax(fabs(xi.x), fabs(xi.y)), fabs(xi.z));
@@ -914,12 +917,12 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
             dx = fma(-L, rint(dx * invL), dx);
             dy = fma(-L, rint(dy * invL), dy);
             dz = fma(-L, rint(dz * invL), dz);
-            near = fma(dz, dz, fma(dy, dy, dx * dx)) < rmax2;
+            near = !(fma(dz, dz, fma(dy, dy, dx * dx)) >= rmax2);
         } else {
             const float4 pj = S.jf[k];
             const float dx = pj.x - xf, dy = pj.y - yf, dz = pj.z - zf;
             const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            near = r2 < thr;
+            near = !(r2 >= thr);
             if (CHECK) far |= r2 >= hl2 ? 1u << k : 0u;
         }
         nm |= near ? 1u << k : 0u;
@@ -928,7 +931,7 @@ __device__ __forceinline__ bool nb_chunk_f64(const Dev& d, const Rep& R, RepStat
         __syncwarp();  // the staged entries have been read
         return false;
     }
-    nm = (nm | odd) & col;
+    nm &= col;
     const uint32_t below = (1u << lane) - 1u;
     const double us = COUL ? 2.0 / R.rc_c2 : 0.0;
     const double2* lj = d.lj64 + R.lj_off;
