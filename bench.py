@@ -50,6 +50,7 @@ sys.path.insert(0, ROOT)
 L2_FLUSH_BYTES = 256 << 20          # > 126 MB L2: each timed step starts with a cold L2
 MEASURED_PEAK_HBM_GBS = 6538.9      # fallback when MEASURED_PEAKS.json is absent: measured copy BW
 SM_COUNT, FP32_LANES = 148, 128
+STATE_RECORD = 304                  # bytes of a replica's state record (RepState), read after every call
 WORKLOADS = ("water30k", "argon4k", "water750k", "batch256", "serve")
 CPU_MAX_ATOMS = 100_000             # above this the reference's O(N^2) list build takes hours
 
@@ -379,7 +380,7 @@ def run_single(args, R: Ranks):
                       "mixed_over_fp64": round(value / value64, 3)},
         "accuracy_vs_fp64_cpu_oracle": acc,
         "e2e": {"value": round(e2e_value, 1), "unit": "atom-steps/s",
-                "h2d_bytes_per_step": 8, "d2h_bytes_per_step": 8 + 2 * 232,
+                "h2d_bytes_per_step": 8, "d2h_bytes_per_step": STATE_RECORD,
                 "how": "Engine.run_n(1) + Engine.potential_energy per MD step (C ABI, host "
                        "buffers, host wall clock); inputs are the step target, result the "
                        "energy scalars"},
@@ -562,9 +563,9 @@ def run_batch(args, R: Ranks):
                                   "graph per step), device step times summed over the replicas"},
         "accuracy_vs_fp64_cpu_oracle": acc,
         "e2e": {"value": round(e2e_value, 1), "unit": "atom-steps/s", "steps": n_e2e,
-                "h2d_bytes_per_step": 4, "d2h_bytes_per_step": 240 * len(cfgs),
+                "h2d_bytes_per_step": 4, "d2h_bytes_per_step": STATE_RECORD * len(cfgs),
                 "how": "Batch.step(1) per MD step through the C ABI (returns after the device "
-                       "finished; reads back each replica's 240-byte status record), potential "
+                       f"finished; reads back each replica's {STATE_RECORD}-byte state record), potential "
                        "energies of all replicas read at the end; host wall clock"},
         "roofline": roof,
         "cpu_baseline": cpu,

@@ -316,8 +316,8 @@ class Engine:
 
     def launch_info(self) -> dict:
         """The launch configuration of the device table (valid after a step):
-        pair-kernel form, blocks per SM the autotuner chose, whether the
-        minimum-image pair kernel runs, kernels per captured step."""
+        pair-kernel form, its blocks per SM, whether the minimum-image pair
+        kernel runs, kernels per captured step."""
         info = _capi.dmdgpu_launch_info()
         self._check(self._lib.dmdgpu_get_launch_info(self._h, C.byref(info)))
         return _capi.launch_info_dict(info)

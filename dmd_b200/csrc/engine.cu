@@ -142,7 +142,7 @@ void sort_grid(int n, double L, int& nvx, int& nvz) {
 //   P(r^2) = erf(a r) / r^3 - 2 a / sqrt(pi) exp(-a^2 r^2) / r^2
 //          = a^3 (4 / sqrt(pi)) int_0^1 t^2 exp(-a^2 r^2 t^2) dt,
 // by Chebyshev interpolation in extended precision; false when EWALD_N of them
-// do not reach FP64 rounding (a rc above about 3.3) or the cutoff is not usable.
+// do not reach FP64 rounding (a rc above about 3.55) or the cutoff is not usable.
 static bool ewald_polynomial(double alpha, double rc, double* out) {
     using ld = long double;
     constexpr int N = EWALD_N;
@@ -212,8 +212,8 @@ std::mutex g_tune_mu;
 std::map<TuneKey, TuneChoice> g_tune;
 constexpr size_t kStatePiece = 65536;       // atoms of a state copied through the staging block at a time
 constexpr int kTuneSteps = 6;               // timed steps per candidate
-// (only tables with a PME chain are tuned; 4 blocks per SM, for LJ-only tables,
-// come from the rule)
+// (tuned are tables of one system with a PME chain, and those of the cluster form;
+// 4 blocks per SM, for LJ-only tables, come from the rule)
 constexpr TuneChoice kTuneCand[] = {{NB_CLUSTER8, 1}, {NB_CLUSTER8, 2}, {NB_CHUNK32, 1}, {NB_CHUNK32, 2},
                                     {NB_CHUNK32, 3}};
 
@@ -1557,7 +1557,8 @@ void Batch::drop_graphs() {
 // Capturing and instantiating costs 0.3-1 ms, what it saves in 60 to 300
 // steps, so it waits until a table has run 256: a served table that is rebuilt
 // every few calls keeps the one-step graph (at 64 a served wave of 8 jobs took
-// 120.5 ms against 116.0).
+// 120.5 ms against 116.0).  Decided once per call, from the steps of the calls
+// before it: a first call stays with the one-step graph, however long.
 constexpr int kManySteps = 4;
 constexpr int kRefCycle = 5;  // REF: the steps from one list rebuild to the next
 constexpr int kManyAfter = 256;

@@ -15,8 +15,10 @@
 //    offset rounded once per j, FP32 arithmetic; a pair whose r^2 lies within
 //    1e-5 relative of a cutoff is re-tested with the FP64 reference expression,
 //    so the interacting set is exactly the reference's.
-//  * fp64: unwrapped FP64 coordinates with the reference's minimum image and
-//    LJ operation order, no FMA contraction in the per-pair force.
+//  * fp64: FP64 coordinates in the list's image where that is the nearest one
+//    (nb_chunk_f64), the nearest image per pair elsewhere; FP64 arithmetic with
+//    FMA, within rounding of the reference's expressions; a pair within 1e-12
+//    relative of a cutoff is re-tested with the reference's expression.
 #include <algorithm>
 
 #include "device.cuh"
@@ -706,7 +708,8 @@ struct ChunkStage64 {
 };
 
 // One chunk of a replica whose Ewald polynomial does not apply (alpha rc beyond
-// what EWALD_N coefficients reach): erfc() and exp() for the real-space Ewald
+// what EWALD_N coefficients reach, about 3.55; water 30k at 3.74: 539 us per step
+// against 200 at 3.12): erfc() and exp() for the real-space Ewald
 // term, LJ in the reference's operation order, the minimum image taken per pair
 // with the reference's expression.
 __device__ __noinline__ void nb_chunk_f64_erfc(const Dev& d, const Rep& R, RepState* s, int c, int lane, ChunkStage64& S,
@@ -812,7 +815,8 @@ __device__ __forceinline__ double rsqrt_h(double x) {
 // the pairs are found first (single precision, against a bound no pair inside
 // exceeds), listed, and spread evenly over the lanes; their forces go to shared
 // memory, from which each lane sums those on its own entry and atom in the
-// list's order.  Water 30k, 22,800 chunks: 178 -> 139 us per launch, 25 % of
+// list's order.  Water 30k, 22,800 chunks: 178 -> 139 us per launch (140 with
+// non-finite coordinates noticed), 25 % of
 // the FP64 pipe's cycles and 70 % of the L1 / shared data path's; three blocks per SM (80
 // registers, spills) 161 us, the coefficients in registers (spills) 164 us,
 // a pair's force over r instead of its components 153 us, one pair a turn instead

@@ -9,9 +9,14 @@ namespace dmd {
 
 // Launch with programmatic stream serialisation: the kernel may be set up on the
 // device while the kernel before it in the stream still runs, and waits for
-// that kernel's completion in its own chain_wait() (device.cuh).  Every kernel
-// launched this way calls chain_wait() before it touches memory.  Saves about
+// that kernel's completion in its own chain_wait() (device.cuh).  Saves about
 // 1 us of launch latency per kernel of the step's chain.
+// The rule for such a kernel: every thread that stays calls chain_wait(); before
+// it, a kernel stores nothing and loads only what the kernel directly before it
+// does not write (k_kick_drift, k_shake, k_kick2, k_rattle, k_replica_update and
+// k_pme_convert load ahead; the others call it first).  Whatever ran earlier is
+// complete by then: chain_wait() lets the next kernel be set up only after its
+// own wait, so a kernel's blocks start when the one two before it has ended.
 template <typename... P, typename... A>
 inline void launch_chained_smem(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};

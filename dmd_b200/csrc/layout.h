@@ -119,6 +119,7 @@ struct RepState {
     double dr_L;          // box edge before that scale
     int dr_move;          // the replica advances
 };
+static_assert(sizeof(RepState) == 304, "bench.py counts the bytes of this record (STATE_RECORD)");
 
 // Kernel view of the whole batch (passed by value).
 struct Dev {
